@@ -19,6 +19,25 @@ def _rn(g, *s):
     return torch.randn(*s, generator=g, device="cuda")
 
 
+# sorted aggregates of half and fp32 values: the same sums bit for bit as the kernel without a workspace
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("L,D,M,K", [(128, 64, 1, 128), (390, 128, 2, 256), (1024, 64, 3, 64), (640, 128, 1, 1024)])
+def test_sorted_aggregates_of_half_and_fp32_values(api, dtype, L, D, M, K):
+    g = _gen(L * 3 + K)
+    v = _rn(g, 2, L, 2, D).to(dtype).transpose(1, 2)
+    codes = torch.randint(0, K, (2, 2, L, M), generator=g, device="cuda", dtype=torch.int32)
+    codes[:, 1, : L // 2] = 5                                   # more keys of one code than a warp stages at once
+    nb = L // 128
+    want = api.build_aggregates(codes, v, K, nb, impl="scan")
+    got = api.build_aggregates(codes, v, K, nb, state_blocks=nb)
+    api.check_status()
+    for a, b in zip(got[:2], want):
+        assert torch.equal(a, b)
+    cnt, vs = torch.zeros_like(got[2]), torch.zeros_like(got[3])
+    api.cache_advance(codes[:, :, : nb * 128], v[:, :, : nb * 128], K, cnt, vs)
+    assert torch.equal(got[2], cnt) and torch.equal(got[3], vs)
+
+
 # rows gathered as 16-byte vectors (64, 128, 256, 512 bytes a row; the first falls back to single elements), indexes outside the array
 @pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 32), (torch.bfloat16, 64), (torch.float16, 128), (torch.float32, 128)])
 @pytest.mark.parametrize("idx", [torch.int64, torch.int32])

@@ -206,7 +206,9 @@ build_aggregates_reg_kernel(const void *__restrict__ codes, int code_dtype, int6
 //   start[K + 1] u8   start[c] = number of keys with a code below c
 // and a warp of build_aggregates_sorted_kernel reads nine bytes of `start` and the entries between them - no scan,
 // no ballots - and adds row by row (the rows of one code are contiguous, so there is no dispatch on the row either).
-// The sums are formed in the same order as above: bit-identical results.
+// The sums are formed in the same order as above: bit-identical results.  Half and fp32 values take this path as well
+// (B1 H32 D128 L5001, one codebook of 1024, half, with the state: 56 + 11 us; the shared-memory kernel of aggregate.cu and a
+// cache-advance pass over the whole sequence for the state: 129 + 428 us).
 constexpr int kSortWarps = 4;
 
 __host__ __device__ inline int64_t sorted_record_bytes(int64_t K) { return (kBlock + K + 1 + 15) / 16 * 16; }
@@ -277,11 +279,47 @@ sort_block_codes_kernel(const void *__restrict__ codes, int code_dtype, int64_t 
     }
 }
 
-template <int D, bool kState>
+// What a lane of the sorted kernel moves: CPL consecutive elements of a row, 4, 8 or 16 bytes.
+template <int BYTES> __device__ __forceinline__ void ar_copy_async(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+template <int WORDS> __device__ __forceinline__ void ar_load_words(uint32_t addr, uint32_t (&w)[WORDS])
+{
+    if constexpr (WORDS == 4) asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr));
+    else if constexpr (WORDS == 2) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(addr));
+    else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[0]) : "r"(addr));
+}
+template <int WORDS> __device__ __forceinline__ void ar_store_words(void *dst, const uint32_t (&w)[WORDS])
+{
+    if constexpr (WORDS == 4) __stcs(static_cast<uint4 *>(dst), make_uint4(w[0], w[1], w[2], w[3]));
+    else if constexpr (WORDS == 2) __stcs(static_cast<uint2 *>(dst), make_uint2(w[0], w[1]));
+    else __stcs(static_cast<uint32_t *>(dst), w[0]);
+}
+// element e of packed words as fp32, and back
+template <typename T> struct ArElem;
+template <> struct ArElem<__nv_bfloat16> {
+    template <int W> static __device__ __forceinline__ float get(const uint32_t (&w)[W], int e) { return __uint_as_float(e & 1 ? w[e >> 1] & 0xffff0000u : w[e >> 1] << 16); }
+    template <int W> static __device__ __forceinline__ uint32_t word(const float *x, int i) { return Pair16<__nv_bfloat16>::pack(x[2 * i], x[2 * i + 1]); }
+};
+template <> struct ArElem<__half> {
+    template <int W> static __device__ __forceinline__ float get(const uint32_t (&w)[W], int e)
+    {
+        const float2 f = Pair16<__half>::unpack(w[e >> 1]);
+        return e & 1 ? f.y : f.x;
+    }
+    template <int W> static __device__ __forceinline__ uint32_t word(const float *x, int i) { return Pair16<__half>::pack(x[2 * i], x[2 * i + 1]); }
+};
+template <> struct ArElem<float> {
+    template <int W> static __device__ __forceinline__ float get(const uint32_t (&w)[W], int e) { return __uint_as_float(w[e]); }
+    template <int W> static __device__ __forceinline__ uint32_t word(const float *x, int i) { return __float_as_uint(x[i]); }
+};
+
+template <typename T, int D, bool kState>
 __global__ void __launch_bounds__(kArWarps * 32, 7)
-build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const __nv_bfloat16 *__restrict__ v, int64_t v_sb, int64_t v_sh, int v_row_bytes,
+build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const T *__restrict__ v, int64_t v_sb, int64_t v_sh, int v_row_bytes,
                                float *__restrict__ cnt,           // [B,Hkv,NB,MK] dense
-                               __nv_bfloat16 *__restrict__ vsum,  // [B,Hkv,NB,MK,D] dense
+                               T *__restrict__ vsum,              // [B,Hkv,NB,MK,D] dense
                                float *__restrict__ state_cnt,     // nullptr or [B,Hkv,MK]: counts after NBT blocks
                                float *__restrict__ state_vsum,    // nullptr or [B,Hkv,MK,D]: fp32 sums after NBT blocks
                                int Hkv, int M, int K, int NB, int NBT_arg)
@@ -291,6 +329,7 @@ build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const __nv_bfloat
     // (kState = false: NBT = NB and no state - the loop below then has no test on the block index.)
     const int NBT = kState ? NBT_arg : NB;
     constexpr int CPL = D / 32;  // columns per lane: 4 (D = 128) or 2 (D = 64)
+    constexpr int LB = CPL * sizeof(T), W = LB / 4, RB = D * sizeof(T);   // bytes and words per lane, bytes per row
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int MK = M * K;
@@ -303,7 +342,7 @@ build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const __nv_bfloat
     const uint8_t *vblk = reinterpret_cast<const uint8_t *>(v + b * v_sb + h * v_sh + CPL * lane);
     const uint8_t *rec = ws + (static_cast<int64_t>(u) * NBT * M + m) * rec_bytes;
     const int rec_step = M * rec_bytes, v_step = kBlock * v_row_bytes;
-    __nv_bfloat16 *dst = vsum + (static_cast<int64_t>(u) * NB * MK + base) * D + CPL * lane;
+    T *dst = vsum + (static_cast<int64_t>(u) * NB * MK + base) * D + CPL * lane;
     float *cdst = cnt + static_cast<int64_t>(u) * NB * MK + base + lane;
 
     float acc[kArRows][CPL];
@@ -313,24 +352,14 @@ build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const __nv_bfloat
         for (int c = 0; c < CPL; ++c) acc[r][c] = 0.f;
     float my_cnt = 0.f;  // lane r < 8: number of keys of row r so far
 
-    __shared__ __align__(16) uint8_t s_stage[kArWarps][2][kArSlots][D * 2];
-    const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(&s_stage[threadIdx.x >> 5][0][0][0])) + CPL * 2 * lane;
-    auto copy_row = [&](const uint8_t *src, int buf, int slot) {
-        const uint32_t d = stage + (buf * kArSlots + slot) * (D * 2);
-        if constexpr (CPL == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-    };
+    __shared__ __align__(16) uint8_t s_stage[kArWarps][2][kArSlots][RB];
+    const uint32_t stage = static_cast<uint32_t>(__cvta_generic_to_shared(&s_stage[threadIdx.x >> 5][0][0][0])) + LB * lane;
+    auto copy_row = [&](const uint8_t *src, int buf, int slot) { ar_copy_async<LB>(stage + (buf * kArSlots + slot) * RB, src); };
     auto add_slot = [&](float (&a)[CPL], int buf, int slot) {
-        const uint32_t sp = stage + (buf * kArSlots + slot) * (D * 2);
-        uint32_t x0, x1 = 0;
-        if constexpr (CPL == 4) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(x0), "=r"(x1) : "r"(sp));
-        else asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x0) : "r"(sp));
-        a[0] = __fadd_rn(a[0], __uint_as_float(x0 << 16));
-        a[1] = __fadd_rn(a[1], __uint_as_float(x0 & 0xffff0000u));
-        if constexpr (CPL == 4) {
-            a[2] = __fadd_rn(a[2], __uint_as_float(x1 << 16));
-            a[3] = __fadd_rn(a[3], __uint_as_float(x1 & 0xffff0000u));
-        }
+        uint32_t w[W];
+        ar_load_words<W>(stage + (buf * kArSlots + slot) * RB, w);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) a[c] = __fadd_rn(a[c], ArElem<T>::template get<W>(w, c));
     };
     // lane r <= 8: start[row0 + r] of a block's record (the other lanes repeat the last one)
     auto load_start = [&](const uint8_t *rc) { return static_cast<int>(__ldg(rc + kBlock + row0 + (lane < kArRows ? lane : kArRows))); };
@@ -401,10 +430,10 @@ build_aggregates_sorted_kernel(const uint8_t *__restrict__ ws, const __nv_bfloat
         if (!kState || n < NB) {
 #pragma unroll
             for (int r = 0; r < kArRows; ++r) {
-                if constexpr (CPL == 4)
-                    __stcs(reinterpret_cast<uint2 *>(dst + r * D), make_uint2(ar_pack(acc[r][0], acc[r][1]), ar_pack(acc[r][2], acc[r][3])));
-                else
-                    __stcs(reinterpret_cast<uint32_t *>(dst + r * D), ar_pack(acc[r][0], acc[r][1]));
+                uint32_t w[W];
+#pragma unroll
+                for (int i = 0; i < W; ++i) w[i] = ArElem<T>::template word<W>(acc[r], i);
+                ar_store_words<W>(dst + r * D, w);
             }
             if (lane < kArRows) __stcs(cdst, my_cnt);
         }
@@ -433,11 +462,13 @@ size_t aggregates_sorted_workspace_bytes(int64_t B, int64_t Hkv, int64_t NB, int
     return static_cast<size_t>(B * Hkv * NB * M * sorted_record_bytes(K));
 }
 
-// bf16 values and snapshots, D = 64 or 128, K a multiple of 8 and at most 2^15 (shared memory of the sort), rows of v
-// less than 16 MB apart (32-bit offsets inside a block)
+// values and snapshots of one type (bf16, half, fp32), D = 64 or 128, K a multiple of 8 and at most 2^12 (shared memory of
+// the sort), a block's rows of v within 2 GB (32-bit offsets inside a block)
 bool aggregates_sorted_eligible(const VqTensorDesc *v, const VqTensorDesc *vsum, int K)
 {
-    return aggregates_reg_eligible(v, vsum, K) && K <= 4096 && v->stride[2] * 2 * kBlock < (int64_t(1) << 31);
+    const int64_t D = v->shape[3];
+    return v->dtype == vsum->dtype && (D == 64 || D == 128) && K % kArRows == 0 && K <= 4096 &&
+           v->stride[2] * (v->dtype == VQ_F32 ? 4 : 2) * kBlock < (int64_t(1) << 31);
 }
 
 // state_blocks > 0: the walk covers state_blocks >= NB blocks (records for as many in the workspace) and leaves the fp32 counts
@@ -458,20 +489,22 @@ int launch_aggregates_sorted(const VqTensorDesc *codes, const VqTensorDesc *v, i
                                                                     ws, static_cast<int>(Hkv), static_cast<int>(M), K, static_cast<int>(NBT), status);
     const int64_t warps = M * K / kArRows;
     dim3 grid(static_cast<unsigned>((warps + kArWarps - 1) / kArWarps), static_cast<unsigned>(B * Hkv));
-    const int row_bytes = static_cast<int>(v->stride[2] * 2);
-#define VQ_SORTED(DD, ST)                                                                                                          \
-    build_aggregates_sorted_kernel<DD, ST><<<grid, kArWarps * 32, 0, stream>>>(                                                    \
-        ws, static_cast<const __nv_bfloat16 *>(v->ptr), v->stride[0], v->stride[1], row_bytes, static_cast<float *>(cnt->ptr),    \
-        static_cast<__nv_bfloat16 *>(vsum->ptr), state_cnt, state_vsum, static_cast<int>(Hkv), static_cast<int>(M), K,             \
-        static_cast<int>(NB), static_cast<int>(NBT))
+    const int row_bytes = static_cast<int>(v->stride[2] * (v->dtype == VQ_F32 ? 4 : 2));
     const bool with_state = state_vsum != nullptr;
-    if (D == 64) {
-        if (with_state) VQ_SORTED(64, true);
-        else VQ_SORTED(64, false);
-    } else {
-        if (with_state) VQ_SORTED(128, true);
-        else VQ_SORTED(128, false);
-    }
+#define VQ_SORTED(T, DD, ST)                                                                                                       \
+    build_aggregates_sorted_kernel<T, DD, ST><<<grid, kArWarps * 32, 0, stream>>>(                                                 \
+        ws, static_cast<const T *>(v->ptr), v->stride[0], v->stride[1], row_bytes, static_cast<float *>(cnt->ptr),                \
+        static_cast<T *>(vsum->ptr), state_cnt, state_vsum, static_cast<int>(Hkv), static_cast<int>(M), K, static_cast<int>(NB),   \
+        static_cast<int>(NBT))
+#define VQ_SORTED_T(T)                                                                                                             \
+    if (D == 64 && with_state) VQ_SORTED(T, 64, true);                                                                             \
+    else if (D == 64) VQ_SORTED(T, 64, false);                                                                                     \
+    else if (with_state) VQ_SORTED(T, 128, true);                                                                                  \
+    else VQ_SORTED(T, 128, false)
+    if (v->dtype == VQ_F32) { VQ_SORTED_T(float); }
+    else if (v->dtype == VQ_F16) { VQ_SORTED_T(__half); }
+    else { VQ_SORTED_T(__nv_bfloat16); }
+#undef VQ_SORTED_T
 #undef VQ_SORTED
     return launch_status();
 }
