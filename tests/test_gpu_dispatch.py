@@ -19,6 +19,24 @@ def _rn(g, *s):
     return torch.randn(*s, generator=g, device="cuda")
 
 
+# half and fp32 keys on the tensor cores (two bf16 terms from the start): the same codes as the exact kernel, whole numbers
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("L,D,M,K", [(1, 128, 1, 128), (127, 64, 2, 128), (385, 128, 2, 128), (129, 128, 4, 256), (257, 128, 8, 256), (700, 64, 3, 384),
+                                     (640, 128, 2, 512), (1025, 128, 1, 1024)])
+def test_assign_half_and_fp32_keys_equal_the_exact_kernel(api, dtype, L, D, M, K):
+    g = _gen(L + K)
+    cb = _rn(g, 3, M, K, D) * D ** -0.25
+    cb[:, :, 1::8] = cb[:, :, 0::8] * (1 + 2.0 ** -18)        # near-twins: inside the bound of the approximate scores
+    for scale in (1.0, 300.0):
+        k = (_rn(g, 2, L, 3, D) * scale).to(dtype)
+        k[:, L // 2] = 0                                       # every score ties
+        k = k.transpose(1, 2)
+        got = api.assign_codes(k, cb, out_dtype=torch.int32)
+        want = api.assign_codes(k, cb, out_dtype=torch.int32, impl="simt")
+        api.check_status()
+        assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
+
+
 # sorted aggregates of half and fp32 values: the same sums bit for bit as the kernel without a workspace
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("L,D,M,K", [(128, 64, 1, 128), (390, 128, 2, 256), (1024, 64, 3, 64), (640, 128, 1, 1024)])

@@ -1,12 +1,13 @@
 // Key -> code assignment with the score matrix on the tensor cores, still bit-exact.
 //
 // Replaces ops/mini_vq.py:4-18 of the reference (and its greedy-residual extension to M codebooks)
-// for bf16 keys.  The defining arithmetic is unchanged: the code of a key in codebook m is the first
+// for bf16, half and fp32 keys.  The defining arithmetic is unchanged: the code of a key in codebook m is the first
 // arg-max over c of the fp32 fused-multiply-add chain  sum_d r_m[d] * C_m[c][d] (+ bias),
 // r_0 = k, r_{m+1} = r_m - C_m[code] (fp32 subtraction).  What changes is how the arg-max is found:
 //   1. APPROXIMATE scores of a 128-key tile against all K codewords come from tcgen05.mma.  The
 //      fp32 codebook is split into two bf16 terms, C = Ch + Cl + eC with |eC| <= 2^-18 |C|.  The
-//      residual is carried as two bf16 terms as well, rho_m = Rh + Rl (rho_0 = k exactly, Rl = 0);
+//      residual is carried as two bf16 terms as well, rho_m = Rh + Rl (bf16 keys: rho_0 = k exactly, Rl = 0; half keys:
+//      rho_0 = k exactly, 8 + 8 >= 11 significant bits; fp32 keys: |rho_0 - k| <= 2^-18 |k|, one more re-split);
 //      after the code of codebook m is known, t = (Rh + Rl) - C_m[code] in fp32 is re-split.  The
 //      tensor cores form  s~ = Rh.Ch + Rl.Ch + Rh.Cl  with fp32 accumulation.
 //   2. Error of s~ against the defining chain, in units of |r| |C| (|r|: the norm of the residual,
@@ -17,7 +18,8 @@
 //      tensor-core accumulation of 3 D (codebook 0: 2 D) exact products, each addition truncated to fp32:
 //      3 D * 2^-23 <= 12 * 2^-18;  index tag in the low five mantissa bits (see tag_score): 2^-18.
 //      Sum for D = 128: 13 units of 2^-18 for codebook 0, 17 + 1.05 m for codebook m; the kernel uses
-//      eps_m = (4 + D/64 + (2 or 3) D/32 + 1.1 m) 2^-18, one unit above that.
+//      eps_m = (4 + D/64 + (2 or 3) D/32 + 1.1 m) 2^-18, one unit above that; with keys that start as two terms (half,
+//      fp32) codebook 0 has three products as well and every codebook one re-split more (1.1 (m + 1)).
 //      A key whose best approximate score leads the runner-up by more than thr = 2 eps |r| max|C_m|
 //      has a unique arg-max: that code is final.
 //   3. The other keys (well under one per cent of the (key, codebook) pairs for random data) keep the
@@ -42,6 +44,10 @@
 // from L2: it needs the warps to hide its latency); one warp issues the MMAs of the streams in turn,
 // so the scan of one stream overlaps the MMAs of the other; one warp issues the TMA loads of the
 // codebook terms (16 KB units, 5-slot ring).  Every wait is bounded.
+// Half keys (B1 H32 D128 L5001, one codebook of 1024): 166 us + repair; on the exact kernel, which half and fp32 keys took
+// before, 1444 us.
+#include <type_traits>
+
 #include "prefill_tc_common.cuh"
 
 namespace vq {
@@ -94,7 +100,7 @@ split_codebook_kernel(const float *__restrict__ cb, __nv_bfloat16 *__restrict__ 
 }
 
 struct AtParams {
-    const __nv_bfloat16 *k;
+    const void *k;       // bf16, half or fp32 rows
     int64_t k_sb, k_sh, k_sl;
     const float *cb;     // [Hkv, M, K, D]
     const float *bias;   // nullptr or [Hkv, M, K]
@@ -171,20 +177,39 @@ __device__ __forceinline__ void load_scores(uint32_t taddr, const float *bm, int
     }
 }
 
+// four residual columns as bf16 hi and lo terms, 8 bytes each, at byte `off` of the two operand tiles
+__device__ __forceinline__ void store_terms(uint8_t *a_rh, uint8_t *a_rl, uint32_t off, const float (&x)[4])
+{
+    uint32_t wh[2], wl[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const __nv_bfloat16 h0 = __float2bfloat16_rn(x[2 * e]), h1 = __float2bfloat16_rn(x[2 * e + 1]);
+        __nv_bfloat162 hv = __halves2bfloat162(h0, h1);
+        wh[e] = *reinterpret_cast<uint32_t *>(&hv);
+        wl[e] = pack_bf16(x[2 * e] - __bfloat162float(h0), x[2 * e + 1] - __bfloat162float(h1));
+    }
+    *reinterpret_cast<uint2 *>(a_rh + off) = make_uint2(wh[0], wh[1]);
+    *reinterpret_cast<uint2 *>(a_rl + off) = make_uint2(wl[0], wl[1]);
+}
+
 // WRAP: a codebook has more chunks than the stream's score region holds and goes through it in rounds.
-template <int D, int NS, int CH, bool WRAP>
+// KT: key type.  bf16 keys are the first residual as they lie in memory (a TMA tile); half and fp32 keys are split into two
+// bf16 terms by the scan warps first (kConv).
+template <typename KT, int D, int NS, int CH, bool WRAP>
 __global__ void __launch_bounds__(AtCfg<D, NS, CH>::kThreads, 1)
 assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_hi,
                  const __grid_constant__ CUtensorMap tm_lo, AtParams p)
 {
     using C = AtCfg<D, NS, CH>;
     constexpr int NH = C::NH, SL = C::kSlots;
+    constexpr bool kConv = !std::is_same<KT, __nv_bfloat16>::value;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t bar_k[NS], bar_q[NS], bar_c[NS][C::kMaxChunks], c_free[NS][C::kMaxChunks], b_full[SL], b_free[SL];
     __shared__ __align__(8) uint64_t x_half[NS][4], x_done[NS][4];   // hand-offs between the two warps of a lane quarter
     __shared__ __align__(16) float4 s_x[NS][kBlock];                  // per key: what its two threads tell each other
     __shared__ __align__(16) float4 s_y[NS][kBlock];                  // ... the rest of it (third best, runner-up's group, flag)
+    __shared__ float s_norm2[kConv ? NS : 1][kConv ? kBlock : 1];     // squared norms of the keys that the scan warps split
     __shared__ uint32_t s_tmem;
     __shared__ int s_err;
 
@@ -233,8 +258,9 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
     if (warp == C::kWarpTma) {
         // ============================================================ TMA producer
         if (lane == 0) {
-            prefetch_tmap(&tm_k); prefetch_tmap(&tm_hi); prefetch_tmap(&tm_lo);
-            for (int s = 0; s < n_act; ++s) {
+            if (!kConv) prefetch_tmap(&tm_k);
+            prefetch_tmap(&tm_hi); prefetch_tmap(&tm_lo);
+            for (int s = 0; s < n_act && !kConv; ++s) {
                 mbar_expect_tx(&bar_k[s], C::kATile);
 #pragma unroll
                 for (int hh = 0; hh < NH; ++hh)
@@ -274,8 +300,9 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             for (int m = 0; m < M && ok; ++m)
                 for (int ch = 0; ch < chunks && ok; ++ch)
                     for (int s = 0; s < n_act && ok; ++s) {
-                        // the residual terms of (s, m): the key tile itself for m = 0, else written by the scan threads
-                        if (ch == 0 && !(m == 0 ? mbar_wait(&bar_k[s], 0, p.wait_limit) : mbar_wait(&bar_q[s], (m - 1) & 1, p.wait_limit))) {
+                        // the residual terms of (s, m): a bf16 key tile itself for m = 0, else written by the scan threads
+                        if (ch == 0 && !(m == 0 && !kConv ? mbar_wait(&bar_k[s], 0, p.wait_limit)
+                                                          : mbar_wait(&bar_q[s], (kConv ? m : m - 1) & 1, p.wait_limit))) {
                             ok = false;
                             break;
                         }
@@ -301,7 +328,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                             for (int k4 = 0; k4 < 4; ++k4)
                                 mma_ss(dcol, d_rh + static_cast<uint64_t>((k4 * 32) >> 4), d_b + static_cast<uint64_t>((k4 * 32) >> 4), idesc,
                                        (rem | k4) ? 1u : 0u);
-                            if (!is_lo && m > 0) {
+                            if (!is_lo && (kConv || m > 0)) {
 #pragma unroll
                                 for (int k4 = 0; k4 < 4; ++k4)
                                     mma_ss(dcol, d_rl + static_cast<uint64_t>((k4 * 32) >> 4), d_b + static_cast<uint64_t>((k4 * 32) >> 4), idesc, 1u);
@@ -329,8 +356,42 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         float4 *xch = &s_x[s][row];
         float rbound;  // |k| + sum of the largest codeword norms so far: a priori bound of the residual's norm
         float rnow;    // bound of the current residual's norm (tighter): see the residual update below
-        bool ok = __all_sync(kAll, mbar_wait(&bar_k[s], 0, p.wait_limit));
-        {
+        bool ok = true;
+        if constexpr (kConv) {
+            // ---- the keys of this stream as two bf16 terms in the operand layout, and their squared norms.  As in the
+            // residual update below a warp walks 16 of its quarter's keys, D/4 lanes per key: whole rows per load.
+            constexpr int LPR = D / 4, KPI = 32 / LPR, NIT = 16 / KPI;
+            const int sub = lane / LPR, l = lane % LPR;
+            const uint32_t lane_off = (l >> 4) * kHalfBytes + 8 * (l & 1);
+            const int chunk = (l & 15) >> 1;
+            const KT *kb = static_cast<const KT *>(p.k) + b * p.k_sb + h * p.k_sh + 4 * l;
+#pragma unroll 4
+            for (int i = 0; i < NIT; ++i) {
+                const int r = wq * 32 + 16 * hf + i * KPI + sub;
+                float x[4] = {0.f, 0.f, 0.f, 0.f};
+                if (j0 + r < p.L) {
+                    if constexpr (std::is_same<KT, float>::value) {
+                        const float4 v = __ldg(reinterpret_cast<const float4 *>(kb + (j0 + r) * p.k_sl));
+                        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+                    } else {
+                        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(kb + (j0 + r) * p.k_sl));
+                        const float2 f0 = Pair16<KT>::unpack(v.x), f1 = Pair16<KT>::unpack(v.y);
+                        x[0] = f0.x; x[1] = f0.y; x[2] = f1.x; x[3] = f1.y;
+                    }
+                }
+                store_terms(a_rh, a_rl, lane_off + r * 128 + ((chunk ^ (r & 7)) << 4), x);
+                float ss = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+#pragma unroll
+                for (int off = LPR / 2; off >= 1; off >>= 1) ss += __shfl_xor_sync(kAll, ss, off);
+                if (l == 0) s_norm2[s][r] = ss;
+            }
+            fence_proxy_async_smem();
+            mbar_arrive(&bar_q[s]);
+            ok = __all_sync(kAll, mbar_wait(&bar_q[s], 0, p.wait_limit));   // every warp's part, this row's norm among them
+            rbound = sqrtf(s_norm2[s][row]) * 1.0001f;
+            rnow = rbound;
+        } else {
+            ok = __all_sync(kAll, mbar_wait(&bar_k[s], 0, p.wait_limit));
             // |k| from the key tile the TMA load put into shared memory (this thread's row, 16-byte chunks in the
             // 128-byte swizzle: eight consecutive rows read eight different chunks, so the reads do not collide)
             float ss = 0.f;
@@ -352,7 +413,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         for (int m = 0; m < M && ok; ++m) {
             const float cm = p.cmax[h * M + m];
             // eps of this codebook in units of 2^-18: the terms listed at the top of the file plus one unit of slack
-            const float eps_m = (4.f + D / 64 + (m > 0 ? 3 : 2) * (D / 32) + 1.1f * m) * 3.814697265625e-6f;
+            const int splits = kConv ? m + 1 : m;   // re-splits that the residual has been through
+            const float eps_m = (4.f + D / 64 + (splits > 0 ? 3 : 2) * (D / 32) + 1.1f * splits) * 3.814697265625e-6f;
             const float thr0 = 2.f * eps_m * rnow * cm + 1e-30f;
             const float *bm = p.bias ? p.bias + (static_cast<int64_t>(h) * M + m) * K : nullptr;
             // ---- scan of this thread's groups, chunk by chunk as the tensor pipe finishes them: best and runner-up
@@ -549,27 +611,16 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                         for (int i = 0; i < NB; ++i) {
                             const int r = wq * 32 + 16 * hf + (i0 + i) * KPI + sub;
                             const uint32_t off = lane_off + r * 128 + ((chunk ^ (r & 7)) << 4);
-                            uint2 *ph = reinterpret_cast<uint2 *>(a_rh + off);
-                            uint2 *pl = reinterpret_cast<uint2 *>(a_rl + off);
-                            const uint2 vh = *ph;
+                            const uint2 vh = *reinterpret_cast<const uint2 *>(a_rh + off);
                             float x[4] = {__uint_as_float(vh.x << 16), __uint_as_float(vh.x & 0xffff0000u), __uint_as_float(vh.y << 16),
                                           __uint_as_float(vh.y & 0xffff0000u)};
-                            if (m > 0) {
-                                const uint2 vl = *pl;
+                            if (kConv || m > 0) {
+                                const uint2 vl = *reinterpret_cast<const uint2 *>(a_rl + off);
                                 x[0] += __uint_as_float(vl.x << 16); x[1] += __uint_as_float(vl.x & 0xffff0000u);
                                 x[2] += __uint_as_float(vl.y << 16); x[3] += __uint_as_float(vl.y & 0xffff0000u);
                             }
                             x[0] -= crow4[i].x; x[1] -= crow4[i].y; x[2] -= crow4[i].z; x[3] -= crow4[i].w;
-                            uint32_t wh[2], wl[2];
-#pragma unroll
-                            for (int e = 0; e < 2; ++e) {
-                                const __nv_bfloat16 h0 = __float2bfloat16_rn(x[2 * e]), h1 = __float2bfloat16_rn(x[2 * e + 1]);
-                                __nv_bfloat162 hv = __halves2bfloat162(h0, h1);
-                                wh[e] = *reinterpret_cast<uint32_t *>(&hv);
-                                wl[e] = pack_bf16(x[2 * e] - __bfloat162float(h0), x[2 * e + 1] - __bfloat162float(h1));
-                            }
-                            *ph = make_uint2(wh[0], wh[1]);
-                            *pl = make_uint2(wl[0], wl[1]);
+                            store_terms(a_rh, a_rl, off, x);
                         }
                     }
                 }
@@ -584,7 +635,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 const float c2 = __ldg(p.cn2 + static_cast<int64_t>(h) * MK + m * K + code);
                 const float slack = 2.f * eps_m * rnow * cm + (bm ? fabsf(best) * 4.76837158203125e-7f : 0.f);
                 const float ss = fmaxf(rnow * rnow - 2.f * (s_code - slack) + c2, 0.f);
-                rnow = sqrtf(ss) * 1.001f + static_cast<float>(m + 1) * 7.7e-6f * rbound;
+                rnow = sqrtf(ss) * 1.001f + static_cast<float>(splits + 1) * 7.7e-6f * rbound;
                 fence_proxy_async_smem();
                 tc_fence_before();
                 mbar_arrive(&bar_q[s]);
@@ -620,7 +671,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 // per candidate runs the chain; without one (too many candidates, no room for the record, or a code of
 // an earlier codebook has changed and with it the residual) lane l scores the codes l, l + 32, ... of
 // the whole codebook.  The residual is broadcast from shared memory.
-template <int D>
+template <typename KT, int D>
 __global__ void __launch_bounds__(kAtRepairWarps * 32)
 assign_repair_kernel(AtParams p)
 {
@@ -637,7 +688,7 @@ assign_repair_kernel(AtParams p)
         const int64_t lin = static_cast<int64_t>((static_cast<unsigned long long>(ent.y) << 32) | ent.x);
         const int64_t u = lin / p.L, j = lin % p.L;
         const int b = static_cast<int>(u / p.Hkv), h = static_cast<int>(u % p.Hkv);
-        const __nv_bfloat16 *krow = p.k + b * p.k_sb + h * p.k_sh + j * p.k_sl;
+        const KT *krow = static_cast<const KT *>(p.k) + b * p.k_sb + h * p.k_sh + j * p.k_sl;
         const float *cbh = p.cb + static_cast<int64_t>(h) * M * K * D;
         __syncwarp();
         // the key's records, newest first, into a table indexed by codebook
@@ -650,7 +701,7 @@ assign_repair_kernel(AtParams p)
             }
         }
 #pragma unroll
-        for (int i = 0; i < PER; ++i) r[lane + 32 * i] = __bfloat162float(krow[lane + 32 * i]);
+        for (int i = 0; i < PER; ++i) r[lane + 32 * i] = to_f32(krow[lane + 32 * i]);
         __syncwarp();
         const int64_t cbase = b * p.c_sb + h * p.c_sh + j * p.c_sl;
         bool changed = false;
@@ -739,7 +790,7 @@ assign_repair_kernel(AtParams p)
     }
 }
 
-template <int D, int NS, int CH, bool WRAP = false>
+template <typename KT, int D, int NS, int CH, bool WRAP = false>
 static int launch_assign_tc(const VqTensorDesc *k, const VqTensorDesc *cb, const VqTensorDesc *bias, VqTensorDesc *codes,
                             void *workspace, int32_t *status, cudaStream_t stream)
 {
@@ -760,9 +811,11 @@ static int launch_assign_tc(const VqTensorDesc *k, const VqTensorDesc *cb, const
     CUtensorMap mk, mhi, mlo;
     const uint64_t cd[3] = {static_cast<uint64_t>(D), static_cast<uint64_t>(Hkv * MK), 1};
     const uint64_t cs[3] = {1, static_cast<uint64_t>(D), static_cast<uint64_t>(Hkv * MK * D)};
-    if (!map_bhld(&mk, *k) || !make_map(&mhi, hi, 3, cd, cs, CH) || !make_map(&mlo, lo, 3, cd, cs, CH)) return VQ_ELAUNCH;
+    const bool tile = k->dtype == VQ_BF16;   // the other key types are read by the scan warps
+    if ((tile && !map_bhld(&mk, *k)) || !make_map(&mhi, hi, 3, cd, cs, CH) || !make_map(&mlo, lo, 3, cd, cs, CH)) return VQ_ELAUNCH;
+    if (!tile) mk = mhi;
     AtParams p{};
-    p.k = static_cast<const __nv_bfloat16 *>(k->ptr);
+    p.k = k->ptr;
     p.k_sb = k->stride[0]; p.k_sh = k->stride[1]; p.k_sl = k->stride[2];
     p.cb = static_cast<const float *>(cb->ptr);
     p.bias = bias ? static_cast<const float *>(bias->ptr) : nullptr;
@@ -781,7 +834,7 @@ static int launch_assign_tc(const VqTensorDesc *k, const VqTensorDesc *cb, const
     p.wait_limit = wait_limit_cycles();
     static_assert(!WRAP || CH == AtCfg<D, NS, CH>::kRegion, "rounds of one chunk per use of the region");
     if (WRAP != (K / CH > C::kMaxChunks)) return VQ_EUNSUPPORTED;
-    auto kern = assign_tc_kernel<D, NS, CH, WRAP>;
+    auto kern = assign_tc_kernel<KT, D, NS, CH, WRAP>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kTotal) != cudaSuccess) return VQ_ELAUNCH;
     dim3 grid(static_cast<unsigned>((p.ntiles + NS - 1) / NS), static_cast<unsigned>(B * Hkv));
     kern<<<grid, C::kThreads, C::kTotal, stream>>>(mk, mhi, mlo, p);
@@ -789,7 +842,7 @@ static int launch_assign_tc(const VqTensorDesc *k, const VqTensorDesc *cb, const
     // the doubtful keys, exactly; the list length is only known on the device: a fixed grid walks it
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return VQ_EDEVICE;
-    assign_repair_kernel<D><<<static_cast<unsigned>(sms * 8), kAtRepairWarps * 32, 0, stream>>>(p);
+    assign_repair_kernel<KT, D><<<static_cast<unsigned>(sms * 8), kAtRepairWarps * 32, 0, stream>>>(p);
     return launch_status();
 }
 
@@ -813,10 +866,18 @@ extern "C" int vqattn_assign_codes_ws(const VqTensorDesc *k, const VqTensorDesc 
     if (bias != nullptr && bias->ptr == nullptr) bias = nullptr;
     const bool shapes_ok = k->ndim == 4 && codebooks->ndim == 4;
     const int64_t D = shapes_ok ? k->shape[3] : 0, M = shapes_ok ? codebooks->shape[1] : 0, K = shapes_ok ? codebooks->shape[2] : 0;
-    const bool tensor_path = shapes_ok && k->dtype == VQ_BF16 && (D == 64 || D == 128) && M >= 1 && M <= kAtMaxM &&
-                             K % kAtMinChunk == 0 && (K <= 512 || K == kAtMaxK) && k->stride[0] % 8 == 0 && k->stride[1] % 8 == 0 &&
-                             k->stride[2] % 8 == 0 && k->shape[2] < (int64_t(1) << 31);
-    if (!tensor_path) return vqattn_assign_codes(k, codebooks, bias, codes, stream);
+    const int64_t align = k->dtype == VQ_BF16 ? 8 : 4;   // elements: TMA rows, 16- or 8-byte loads of the other key types
+    const bool tensor_path = shapes_ok && is_act_dtype(k->dtype) && (D == 64 || D == 128) && M >= 1 && M <= kAtMaxM &&
+                             K % kAtMinChunk == 0 && (K <= 512 || K == kAtMaxK) && k->stride[0] % align == 0 && k->stride[1] % align == 0 &&
+                             k->stride[2] % align == 0 && k->shape[2] < (int64_t(1) << 31);
+    // Few keys against few codewords: the exact kernel is one launch of a short chain, this path four (codebook split, scan,
+    // repair, a memset).  Measured (us, this path / exact kernel): M*K*D = 8192: 8192 keys 25 / 11, 32768 keys 26 / 25;
+    // 16384: 8192 keys 28 / 17, 32768 keys 28 / 50; 32768: 256 keys 25 / 34, 32768 keys 35 / 84.
+    const bool small = shapes_ok && M * K * D <= (1 << 14) && k->shape[0] * k->shape[1] * k->shape[2] <= (1 << 14);
+    // half and fp32 keys without a (sufficient) workspace take the exact kernel as well
+    const bool ws_ok = workspace != nullptr && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && shapes_ok &&
+                       workspace_bytes >= vqattn_assign_workspace_bytes(k->shape[0], k->shape[1], k->shape[2], M, K, D);
+    if (!tensor_path || small || (k->dtype != VQ_BF16 && !ws_ok)) return vqattn_assign_codes(k, codebooks, bias, codes, stream);
     // same argument checks as the exact kernel's entry point
     int st;
     if ((st = check_basic(k, 4)) != VQ_OK) return st;
@@ -834,26 +895,23 @@ extern "C" int vqattn_assign_codes_ws(const VqTensorDesc *k, const VqTensorDesc 
     if (codes->dtype == VQ_U8 && K > 256) return VQ_EINVAL_DTYPE;
     if (reinterpret_cast<uintptr_t>(k->ptr) % 16 || reinterpret_cast<uintptr_t>(codebooks->ptr) % 16) return VQ_EINVAL_STRIDE;
     if (B * Hkv > 65535) return VQ_EUNSUPPORTED;
-    if (workspace == nullptr || reinterpret_cast<uintptr_t>(workspace) % 256 ||
-        workspace_bytes < vqattn_assign_workspace_bytes(B, Hkv, L, M, K, D))
-        return VQ_EWORKSPACE;
+    if (!ws_ok) return VQ_EWORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // two key tiles per CTA share the 512 score columns of tensor memory when a codebook fits 256 of them;
-    // N = 256 instructions when K is a multiple of 256
-    if (K == 128)
-        return D == 64 ? launch_assign_tc<64, 2, 128>(k, codebooks, bias, codes, workspace, status_word, s)
-                       : launch_assign_tc<128, 2, 128>(k, codebooks, bias, codes, workspace, status_word, s);
-    if (K == 256)
-        return D == 64 ? launch_assign_tc<64, 2, 256>(k, codebooks, bias, codes, workspace, status_word, s)
-                       : launch_assign_tc<128, 2, 256>(k, codebooks, bias, codes, workspace, status_word, s);
-    // K = 512 and K = 1024: two streams, the codebook's 256-column chunks in rounds through each stream's region (the
-    // candidates of a doubtful key are tracked during the scan, the earlier chunks being gone by the end)
-    if (K == 512)
-        return D == 64 ? launch_assign_tc<64, 2, 256, true>(k, codebooks, bias, codes, workspace, status_word, s)
-                       : launch_assign_tc<128, 2, 256, true>(k, codebooks, bias, codes, workspace, status_word, s);
-    if (K == 1024)
-        return D == 64 ? launch_assign_tc<64, 2, 256, true>(k, codebooks, bias, codes, workspace, status_word, s)
-                       : launch_assign_tc<128, 2, 256, true>(k, codebooks, bias, codes, workspace, status_word, s);
-    return D == 64 ? launch_assign_tc<64, 1, 128>(k, codebooks, bias, codes, workspace, status_word, s)   // K = 384
-                   : launch_assign_tc<128, 1, 128>(k, codebooks, bias, codes, workspace, status_word, s);
+    auto go = [&](auto key, auto dim) {
+        using KT = decltype(key);
+        constexpr int DD = decltype(dim)::value;
+        // two key tiles per CTA share the 512 score columns of tensor memory when a codebook fits 256 of them;
+        // N = 256 instructions when K is a multiple of 256
+        if (K == 128) return launch_assign_tc<KT, DD, 2, 128>(k, codebooks, bias, codes, workspace, status_word, s);
+        if (K == 256) return launch_assign_tc<KT, DD, 2, 256>(k, codebooks, bias, codes, workspace, status_word, s);
+        // K = 512 and K = 1024: two streams, the codebook's 256-column chunks in rounds through each stream's region (the
+        // candidates of a doubtful key are tracked during the scan, the earlier chunks being gone by the end)
+        if (K == 512 || K == 1024) return launch_assign_tc<KT, DD, 2, 256, true>(k, codebooks, bias, codes, workspace, status_word, s);
+        return launch_assign_tc<KT, DD, 1, 128>(k, codebooks, bias, codes, workspace, status_word, s);   // K = 384
+    };
+    using D64 = std::integral_constant<int, 64>;
+    using D128 = std::integral_constant<int, 128>;
+    if (k->dtype == VQ_F32) return D == 64 ? go(float(), D64()) : go(float(), D128());
+    if (k->dtype == VQ_F16) return D == 64 ? go(__half(), D64()) : go(__half(), D128());
+    return D == 64 ? go(__nv_bfloat16(), D64()) : go(__nv_bfloat16(), D128());
 }
