@@ -257,7 +257,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 
     if (warp == C::kWarpTma) {
         // ============================================================ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             if (!kConv) prefetch_tmap(&tm_k);
             prefetch_tmap(&tm_hi); prefetch_tmap(&tm_lo);
             for (int s = 0; s < n_act && !kConv; ++s) {
@@ -290,7 +290,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         }
     } else if (warp == C::kWarpMma) {
         // ============================================================ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16(128, CH, 0, 0, 0);
             // descriptors differ only in their 16-byte-granular start address: build the bases once
             const uint64_t d_a0 = smem_desc_sw128(smem_u32(smem), 16, 1024);

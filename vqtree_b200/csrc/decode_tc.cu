@@ -130,7 +130,8 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
 
     // The producer lane initialises the barriers itself and starts the first tile loads at once; the
     // other roles see the barriers after the CTA-wide barrier below (TMEM is allocated meanwhile).
-    if (tid == 5 * 32) {
+    const bool producer = warp == 5 && elect_one();
+    if (producer) {
         for (int i = 0; i < NS; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
@@ -198,7 +199,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
                 dt_bulk_copy(cnt_s + st * kDtRows, p.cnt + static_cast<int64_t>(ue) * p.MK + it.row0, kDtRows * 4, &full[st]);
         }
     };
-    if (tid == 5 * 32) produce(min(n_items, NS));   // the ring is empty: no wait inside
+    if (producer) produce(min(n_items, NS));   // the ring is empty: no wait inside
     if (warp == 4) {
         __syncwarp();
         tmem_alloc(&s_tmem, 64);
@@ -211,13 +212,13 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
 
     if (warp == 5) {
         // ================================================================== producer (the first loads were issued above)
-        if (lane == 0) {
+        if (producer) {
             produce(n_items);
             if (!pr_ok) s_err = 1;
         }
     } else if (warp == 4) {
         // ================================================================== MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = idesc_bf16(128, kDtN, 0, 0);   // S^T = Ktile (K-major) . Q^T (K-major)
             constexpr uint32_t idesc_o = idesc_bf16(128, kDtN, 1, 0);   // O^T = Vtile^T (MN-major A) . P (K-major)
             const uint64_t d_ring = smem_desc_sw128(smem_u32(smem), 16, 1024);

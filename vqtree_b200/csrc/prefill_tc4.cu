@@ -167,7 +167,7 @@ prefill_tc4_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
 
     if (warp == C::kWarpTma) {
         // ================================================================== TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_tmap(&tm_q1); prefetch_tmap(&tm_k1); prefetch_tmap(&tm_v);
             mbar_expect_tx(&bar_q, (p.rerope ? 2 : 1) * C::kTile);
 #pragma unroll
@@ -218,7 +218,7 @@ prefill_tc4_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
         // arithmetic: ring slot, score buffer and their barrier phases are running counters, the operand
         // descriptors of the three slots are built once (only the low word of a descriptor depends on the
         // address), and an item needs the constant-position query exactly when it comes before `n_q2`.
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_qk = idesc_f16kind(128, 128, 0, 0, F16 ? 0u : 1u);
             constexpr uint32_t idesc_pv = idesc_f16kind(128, D, 0, 1, F16 ? 0u : 1u);
             const uint64_t d_q1 = smem_desc_sw128(smem_u32(smem + C::kQ1), 16, 1024);

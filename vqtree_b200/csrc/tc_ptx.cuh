@@ -13,6 +13,17 @@ namespace ptx {
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
+// True in one lane of the (converged) warp.  A branch on elect.sync is known to run in one thread, one on the lane number is
+// not: inside the latter the compiler issues every tcgen05 / TMA instruction through a per-thread loop.  Measured: groups of
+// eight 128x128x16 MMAs with a commit and a satisfied barrier wait each take 512 cycles a group (the full rate) behind
+// elect.sync, 707 - 878 behind `lane == 0`.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
 {
