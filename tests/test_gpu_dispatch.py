@@ -37,6 +37,28 @@ def test_assign_half_and_fp32_keys_equal_the_exact_kernel(api, dtype, L, D, M, K
         assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
 
 
+# keys without a finite error bound (infinities, NaN, squares that overflow) or with a vanishing one (squares that underflow)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,K", [(2, 256), (1, 1024)])
+def test_assign_extreme_keys_equal_the_exact_kernel(api, dtype, M, K):
+    g = _gen(K)
+    cb = _rn(g, 2, M, K, 128) * 128 ** -0.25
+    cb[:, :, 1::8] = cb[:, :, 0::8] * (1 + 2.0 ** -18)
+    k = _rn(g, 2, 2, 400, 128)
+    big, tiny = (3e4, 1e-7) if dtype == torch.float16 else (1e30, 1e-24)
+    k[:, :, 0:8, 3] = float("inf")
+    k[:, :, 8:16, 5] = -float("inf")
+    k[:, :, 16:24, 7] = float("nan")
+    k[:, :, 24:32] = float("nan")
+    k[:, :, 32:128] *= big
+    k[:, :, 128:256] *= tiny
+    k = k.to(dtype)
+    got = api.assign_codes(k, cb, out_dtype=torch.int32)
+    want = api.assign_codes(k, cb, out_dtype=torch.int32, impl="simt")
+    api.check_status()
+    assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
+
+
 # sorted aggregates of half and fp32 values: the same sums bit for bit as the kernel without a workspace
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("L,D,M,K", [(128, 64, 1, 128), (390, 128, 2, 256), (1024, 64, 3, 64), (640, 128, 1, 1024)])

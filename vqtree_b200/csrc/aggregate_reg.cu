@@ -463,11 +463,13 @@ size_t aggregates_sorted_workspace_bytes(int64_t B, int64_t Hkv, int64_t NB, int
 }
 
 // values and snapshots of one type (bf16, half, fp32), D = 64 or 128, K a multiple of 8 and at most 2^12 (shared memory of
-// the sort), a block's rows of v within 2 GB (32-bit offsets inside a block)
+// the sort; half and fp32: the K that the shared-memory kernel takes, so that a workspace never decides what is accepted),
+// a block's rows of v within 2 GB (32-bit offsets inside a block)
 bool aggregates_sorted_eligible(const VqTensorDesc *v, const VqTensorDesc *vsum, int K)
 {
     const int64_t D = v->shape[3];
     return v->dtype == vsum->dtype && (D == 64 || D == 128) && K % kArRows == 0 && K <= 4096 &&
+           (v->dtype == VQ_BF16 || K <= 256 || K % 256 == 0) &&
            v->stride[2] * (v->dtype == VQ_F32 ? 4 : 2) * kBlock < (int64_t(1) << 31);
 }
 

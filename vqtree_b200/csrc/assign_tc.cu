@@ -64,6 +64,9 @@ constexpr int kAtRepairWarps = 4;  // warps per CTA of the repair kernel (one do
 // norm of every codebook (grid.x: codebook, grid.y: slices of kSplitRows rows; cmax zeroed by the launcher, the
 // slices meet in it through an atomic maximum on the bits of their non-negative norms).
 constexpr int kSplitRows = 64;
+// Floor of the squared norms that error bounds are formed from: the squares of elements below 1e-22 vanish in fp32, and a
+// bound of zero would declare every lead safe.
+constexpr float kAtMinNorm2 = 1e-35f;
 __global__ void __launch_bounds__(256)
 split_codebook_kernel(const float *__restrict__ cb, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
                       float *__restrict__ cmax, float *__restrict__ cn2, unsigned int *__restrict__ work_count, int K, int D)
@@ -88,7 +91,7 @@ split_codebook_kernel(const float *__restrict__ cb, __nv_bfloat16 *__restrict__ 
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
         if (lane == 0) cn2[row] = ss;
-        wmax = fmaxf(wmax, sqrtf(ss));
+        wmax = fmaxf(wmax, sqrtf(fmaxf(ss, kAtMinNorm2)));
     }
     if (lane == 0) s_max[warp] = wmax;
     __syncthreads();
@@ -388,7 +391,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             fence_proxy_async_smem();
             mbar_arrive(&bar_q[s]);
             ok = __all_sync(kAll, mbar_wait(&bar_q[s], 0, p.wait_limit));   // every warp's part, this row's norm among them
-            rbound = sqrtf(s_norm2[s][row]) * 1.0001f;
+            rbound = sqrtf(fmaxf(s_norm2[s][row], kAtMinNorm2)) * 1.0001f;
             rnow = rbound;
         } else {
             ok = __all_sync(kAll, mbar_wait(&bar_k[s], 0, p.wait_limit));
@@ -405,7 +408,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     ss = fmaf(x, x, fmaf(y, y, ss));
                 }
             }
-            rbound = sqrtf(ss) * 1.0001f;
+            rbound = sqrtf(fmaxf(ss, kAtMinNorm2)) * 1.0001f;
             rnow = rbound;
         }
         uint32_t doubt = 0;   // bit m: the lead of codebook m's best score did not prove its arg-max (bit 8 + m: no record)
@@ -549,6 +552,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                               (static_cast<uint32_t>(sgrp * 32 + 31 - static_cast<int>(__float_as_uint(second) & 31u)) << 16);
                     }
                     if (wrap && slow) n = 255;
+                    const bool unbounded = !(thr < 3e38f);   // infinities, NaN or an overflowed norm: the approximate scores say nothing
                     const uint32_t gb = (!wrap && slow) ? (gbits | __float_as_uint(o.w)) : 0u;
                     const uint32_t un = __reduce_or_sync(kAll, gb);
 #pragma unroll 1
@@ -576,7 +580,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     if (dflag) {
                         const unsigned int at = atomicAdd(p.counters + 1, 1u);
                         if (at < p.pool_cap) {
-                            p.pool[at] = make_uint4(last_rec, static_cast<uint32_t>(m) | (static_cast<uint32_t>(n > 4 ? 255 : n) << 8), c01, c23);
+                            p.pool[at] = make_uint4(last_rec, static_cast<uint32_t>(m) | (static_cast<uint32_t>(unbounded || n > 4 ? 255 : n) << 8), c01, c23);
                             last_rec = at;
                             doubt |= 1u << m;
                         } else {
@@ -717,6 +721,7 @@ assign_repair_kernel(AtParams p)
                 float bv = -INFINITY;
                 int bi = 0x7fffffff;
                 if (all) {
+                    bi = 0;                                     // no score above -inf (NaN scores): the first code, as in the exact kernel
                     for (int c0 = 0; c0 < K; c0 += 128) {       // four codes per lane at a time: four independent chains
                         float acc[4] = {0.f, 0.f, 0.f, 0.f};
                         const float *row[4];
@@ -877,7 +882,7 @@ extern "C" int vqattn_assign_codes_ws(const VqTensorDesc *k, const VqTensorDesc 
     // half and fp32 keys without a (sufficient) workspace take the exact kernel as well
     const bool ws_ok = workspace != nullptr && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && shapes_ok &&
                        workspace_bytes >= vqattn_assign_workspace_bytes(k->shape[0], k->shape[1], k->shape[2], M, K, D);
-    if (!tensor_path || small || (k->dtype != VQ_BF16 && !ws_ok)) return vqattn_assign_codes(k, codebooks, bias, codes, stream);
+    if (!tensor_path || (small && ws_ok) || (k->dtype != VQ_BF16 && !ws_ok)) return vqattn_assign_codes(k, codebooks, bias, codes, stream);
     // same argument checks as the exact kernel's entry point
     int st;
     if ((st = check_basic(k, 4)) != VQ_OK) return st;
