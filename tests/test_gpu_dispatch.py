@@ -93,3 +93,32 @@ def test_gather_aggregates_moves_whole_rows(api, dtype, D, idx):
         ok = (at >= 0) & (at <= L) & (torch.ones_like(cnt, dtype=torch.bool) if c is None else c > 0)
         want = torch.gather(v, 2, at.clamp(0, L).reshape(B, H, -1, 1).expand(-1, -1, -1, D)).reshape(B, H, NB, C, D)
         assert torch.equal(got, torch.where(ok[..., None], want, torch.zeros_like(want)))
+
+
+# the fp32 kernel (64-row tiles, 64-key chunks) against the one-warp-per-row kernel: edges of tiles, chunks, the window and the
+# boundary block; codes without members whose codeword scores highest; infinities behind weights of zero.  Both are fp32 chains:
+# scores of at most 16 (log2 units) carry D + 2 roundings of 2^-24 at most, sums of n <= 2000 weights as many: 2e-5 is above both.
+@pytest.mark.parametrize("L,W,D,Hq,Hkv,M,K", [(1, 128, 64, 1, 1, 1, 128), (63, 128, 128, 2, 1, 1, 128), (129, 128, 64, 2, 2, 1, 128), (257, 128, 128, 4, 2, 2, 128),
+                                              (320, 128, 64, 3, 1, 1, 128), (449, 256, 64, 2, 1, 2, 256), (833, 128, 128, 2, 2, 1, 384), (1024, 512, 64, 4, 4, 2, 256)])
+@pytest.mark.parametrize("rerope", [False, True])
+def test_prefill_fp32_equals_the_row_kernel(api, L, W, D, Hq, Hkv, M, K, rerope):
+    g = _gen(L + D)
+    q1, q2 = (_rn(g, 2, L, Hq, D).transpose(1, 2) for _ in range(2))
+    k1, k3, v = (_rn(g, 2, Hkv, L, D) for _ in range(3))
+    if not rerope:
+        q2, k3 = q1, k1
+    v[:, :, L - 1, 0] = float("inf")                        # the last key: weight zero in every other row
+    nb = api.far_blocks(L, W)
+    act = cnt = vs = None
+    if nb:
+        act = _rn(g, Hkv, M * K, D) * D ** -0.25
+        act[:, 3] *= 30
+        cnt = torch.randint(0, 4, (2, Hkv, nb, M * K), generator=g, device="cuda").float()
+        cnt[..., 3] = 0
+        vs = _rn(g, 2, Hkv, nb, M * K, D) * cnt[..., None]
+        vs[..., 3, :] = float("inf")
+    got, lse = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True)
+    want, lse_w = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True, impl="simt")
+    assert torch.equal(torch.isinf(got), torch.isinf(want))
+    ok = ~torch.isinf(want)
+    assert (got[ok] - want[ok]).abs().max() < 2e-5 and (lse - lse_w).abs().max() < 2e-5

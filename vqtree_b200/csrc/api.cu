@@ -6,6 +6,7 @@
 
 namespace vq {
 int launch_prefill_simt(const VqPrefillArgs *a, cudaStream_t stream);
+int launch_prefill_f32(const VqPrefillArgs *a, cudaStream_t stream);
 int launch_prefill_tensor4(const VqPrefillArgs *a, cudaStream_t stream);
 }  // namespace vq
 
@@ -133,7 +134,8 @@ extern "C" int vqattn_prefill(const VqPrefillArgs *a, void *stream)
     if (B * Hq > 65535) return VQ_EUNSUPPORTED;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     int impl = a->impl;
-    if (impl == VQ_IMPL_AUTO) impl = is_16bit(dt) ? VQ_IMPL_TENSOR : VQ_IMPL_SIMT;
+    if (impl == VQ_IMPL_AUTO && !is_16bit(dt)) return launch_prefill_f32(a, s);
+    if (impl == VQ_IMPL_AUTO) impl = VQ_IMPL_TENSOR;
     if (impl == VQ_IMPL_SIMT) return launch_prefill_simt(a, s);
     if (impl == VQ_IMPL_TENSOR) {
         if (!is_16bit(dt)) return VQ_EINVAL_DTYPE;
