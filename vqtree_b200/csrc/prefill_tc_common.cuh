@@ -97,27 +97,28 @@ inline bool make_map(CUtensorMap *out, const void *ptr, int rank, const uint64_t
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-inline bool map_bhld(CUtensorMap *out, const VqTensorDesc &t)
+inline bool map_bhld(CUtensorMap *out, const VqTensorDesc &t, int box_rows = kBlock)
 {
     const uint64_t dims[4] = {static_cast<uint64_t>(t.shape[3]), static_cast<uint64_t>(t.shape[2]),
                               static_cast<uint64_t>(t.shape[1]), static_cast<uint64_t>(t.shape[0])};
     const uint64_t str[4] = {1, static_cast<uint64_t>(t.stride[2]), static_cast<uint64_t>(t.stride[1]),
                              static_cast<uint64_t>(t.stride[0])};
-    return make_map(out, t.ptr, 4, dims, str, kBlock, t.dtype == VQ_F16);
+    return make_map(out, t.ptr, 4, dims, str, box_rows, t.dtype == VQ_F16);
 }
 
 struct TcMaps {
     CUtensorMap q1, q2, k1, k3, v, cb, vs;
 };
 
-// Fills the seven tensor maps and the kernel parameters from the C-ABI arguments.
+// Fills the seven tensor maps (kv_rows: rows of a key / value box; the query boxes have 128) and the kernel parameters from
+// the C-ABI arguments.
 template <int D>
-inline int tc_setup(const VqPrefillArgs *a, TcMaps &m, TcParams &p)
+inline int tc_setup(const VqPrefillArgs *a, TcMaps &m, TcParams &p, int kv_rows)
 {
     const int64_t B = a->q1.shape[0], Hq = a->q1.shape[1], L = a->q1.shape[2], Hkv = a->k1.shape[1];
     const bool far = a->codebook.ptr != nullptr && a->cnt.ptr != nullptr;
-    if (!map_bhld(&m.q1, a->q1) || !map_bhld(&m.q2, a->q2) || !map_bhld(&m.k1, a->k1) || !map_bhld(&m.k3, a->k3) ||
-        !map_bhld(&m.v, a->v))
+    if (!map_bhld(&m.q1, a->q1) || !map_bhld(&m.q2, a->q2) || !map_bhld(&m.k1, a->k1, kv_rows) ||
+        !map_bhld(&m.k3, a->k3, kv_rows) || !map_bhld(&m.v, a->v, kv_rows))
         return VQ_ELAUNCH;
     p = TcParams{};
     if (far) {
@@ -126,7 +127,7 @@ inline int tc_setup(const VqPrefillArgs *a, TcMaps &m, TcParams &p)
         const uint64_t cs[3] = {1, static_cast<uint64_t>(D), MK * D};
         const uint64_t vd[3] = {static_cast<uint64_t>(D), MK, static_cast<uint64_t>(B * Hkv) * NB};
         const bool f16 = a->q1.dtype == VQ_F16;
-        if (!make_map(&m.cb, a->codebook.ptr, 3, cd, cs, kBlock, f16) || !make_map(&m.vs, a->vsum.ptr, 3, vd, cs, kBlock, f16))
+        if (!make_map(&m.cb, a->codebook.ptr, 3, cd, cs, kv_rows, f16) || !make_map(&m.vs, a->vsum.ptr, 3, vd, cs, kv_rows, f16))
             return VQ_ELAUNCH;
         p.MK = static_cast<int>(MK);
         p.NB = static_cast<int>(NB);
