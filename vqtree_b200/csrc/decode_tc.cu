@@ -48,8 +48,7 @@ constexpr float kDtLazy = 8.f;
 
 struct DtParams {
     DecodeParams d;
-    int tiles_wi;        // window items per unit (tiles, plus one when a tile straddles n_bd)
-    int ts;              // the straddling tile or -1
+    int tiles_wi, tiles_k3;   // window tiles per unit, and how many of them come first: the rows before n_bd
     int tiles_f, TU, units, num_ctas;
     float *partial;      // [(num_ctas + units)][G][D+2]
     int *ticket;         // [units]
@@ -60,7 +59,7 @@ struct DtParams {
 struct DtItem {
     int kind;            // 0: window rows scored q1.k1, 1: window rows scored q2.k3, 2: far rows (q2.codebook)
     int row0;            // first row of the tile in its source
-    int lo, hi;          // valid rows of the tile: [lo, hi)
+    int hi;              // valid rows of the tile: [0, hi)
 };
 
 __device__ __forceinline__ DtItem dt_item(const DtParams &bp, int tt)
@@ -68,27 +67,15 @@ __device__ __forceinline__ DtItem dt_item(const DtParams &bp, int tt)
     const DecodeParams &p = bp.d;
     DtItem it;
     if (tt < bp.tiles_wi) {
-        int t = tt;
-        bool second = false;
-        if (bp.ts >= 0 && tt > bp.ts) {
-            t = tt - 1;
-            second = tt == bp.ts + 1;
-        }
-        const int r0 = t * kDtRows, r1 = min(r0 + kDtRows, p.n_valid);
-        it.row0 = r0;
-        if (bp.ts >= 0 && t == bp.ts) {
-            it.kind = second ? 0 : 1;
-            it.lo = second ? p.n_bd - r0 : 0;
-            it.hi = second ? r1 - r0 : p.n_bd - r0;
-        } else {
-            it.kind = r0 >= p.n_bd ? 0 : 1;
-            it.lo = 0;
-            it.hi = r1 - r0;
-        }
+        // the rows on either side of n_bd are tiled from their own first row (a TMA box may start at any row), so no
+        // key tile is read twice for the two kinds of rows in it
+        const bool k3 = tt < bp.tiles_k3;
+        it.kind = k3 ? 1 : 0;
+        it.row0 = k3 ? tt * kDtRows : p.n_bd + (tt - bp.tiles_k3) * kDtRows;
+        it.hi = min(kDtRows, (k3 ? p.n_bd : p.n_valid) - it.row0);
     } else {
         it.kind = 2;
         it.row0 = (tt - bp.tiles_wi) * kDtRows;
-        it.lo = 0;
         it.hi = kDtRows;
     }
     return it;
@@ -356,7 +343,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
             tmem_ld16(tmem + lane_off + 16 * sb, sr);
             tc_wait_ld();
             const float w = it.kind == 2 ? cnt_s[st * kDtRows + tid] : 1.f;
-            const bool valid = tid >= it.lo && tid < it.hi && w > 0.f;
+            const bool valid = tid < it.hi && w > 0.f;
             float sc[kDtN];
             bool exceed = false;
 #pragma unroll
@@ -626,9 +613,8 @@ int launch_decode_tc(const VqDecodeArgs *a, const DecodeParams &p, cudaStream_t 
     const int64_t B = a->q1.shape[0], Hq = a->q1.shape[1], Hkv = a->k1_win.shape[1];
     DtParams bp{};
     bp.d = p;
-    const int tiles_w = (p.n_valid + kDtRows - 1) / kDtRows;
-    bp.ts = (p.n_bd % kDtRows != 0 && p.n_bd < p.n_valid) ? p.n_bd / kDtRows : -1;
-    bp.tiles_wi = tiles_w + (bp.ts >= 0 ? 1 : 0);
+    bp.tiles_k3 = (p.n_bd + kDtRows - 1) / kDtRows;
+    bp.tiles_wi = bp.tiles_k3 + (p.n_valid - p.n_bd + kDtRows - 1) / kDtRows;
     bp.tiles_f = p.use_far ? p.MK / kDtRows : 0;
     bp.TU = bp.tiles_wi + bp.tiles_f;
     bp.units = static_cast<int>(B * Hkv);
