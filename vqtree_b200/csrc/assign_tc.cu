@@ -57,6 +57,7 @@ using namespace ptx;
 constexpr int kAtMinChunk = 128;   // codewords per MMA chunk: 128, or 256 (one N = 256 instruction) when K allows
 constexpr int kAtMaxM = 8;
 constexpr int kAtMaxK = 1024;   // 32 groups of 32 codes: one bit each in a thread's group mask
+constexpr unsigned int kAtLeft = 64;
 constexpr int kAtRepairWarps = 4;  // warps per CTA of the repair kernel (one doubtful key per warp at a time)
 
 // ------------------------------------------------------------------------------------------------
@@ -72,7 +73,7 @@ split_codebook_kernel(const float *__restrict__ cb, __nv_bfloat16 *__restrict__ 
                       float *__restrict__ cmax, float *__restrict__ cn2, unsigned int *__restrict__ work_count, int K, int D)
 {
     __shared__ float s_max[8];
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) work_count[threadIdx.x] = 0u;   // the scan kernel that follows fills the lists
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 3) work_count[threadIdx.x] = 0u;   // the scan kernel that follows fills the lists
     const int hm = blockIdx.x;  // h * M + m
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float wmax = 0.f;
@@ -116,10 +117,11 @@ struct AtParams {
     int64_t L;
     int32_t *status;
     long long wait_limit;  // cycles a device-side wait may last before the kernel gives up
-    uint4 *work;                // doubtful keys: {key index lo, hi, last record, doubtful codebooks | brute-force codebooks << 8}
+    uint4 *work;                // doubtful keys: {key index lo, hi, last record, doubtful codebooks | brute-force codebooks << 8};
+                                // from the front those whose candidates are known, from the back the others (one entry per key in all)
     uint4 *pool;                // candidate records: {previous record of the key, m | n << 8, codes 0-1, codes 2-3}
-    unsigned int *counters;     // [0] entries in `work`, [1] records in `pool` (zeroed by split_codebook_kernel)
-    unsigned int pool_cap;
+    unsigned int *counters;     // [0] entries at the front of `work`, [1] records in `pool`, [2] entries at the back (zeroed by split_codebook_kernel)
+    unsigned int pool_cap;      // records in `pool` and entries in `work`: one per key
 };
 
 template <int D, int NS, int CH>
@@ -413,6 +415,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         }
         uint32_t doubt = 0;   // bit m: the lead of codebook m's best score did not prove its arg-max (bit 8 + m: no record)
         uint32_t last_rec = 0xffffffffu;   // the key's most recent candidate record
+        bool heavy = false;                // a whole codebook has to be scored
         for (int m = 0; m < M && ok; ++m) {
             const float cm = p.cmax[h * M + m];
             // eps of this codebook in units of 2^-18: the terms listed at the top of the file plus one unit of slack
@@ -430,7 +433,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             // largest of all group maxima and group runners-up, and whether the runner-up of any group came within the
             // threshold of the running best (the other 30 scores of such a group are unknown here and may hold further
             // candidates).  A doubtful key whose third lies below the cut needs no second look at its scores - which WRAP
-            // could not take anyway: the scores of earlier chunks are gone by then.
+            // could not take anyway: the scores of earlier chunks are gone by then, so there the third of such a group is
+            // looked up at once (M4 K512, 2 x 16384 tokens x 32 heads: 279 -> 115 us of repair, the scan stays at 1.49 ms).
             float third = -INFINITY;
             int sgrp = g_lo;
             bool amb = bm != nullptr;   // with a bias the threshold moves with the best score: no short list then
@@ -455,7 +459,22 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 } else {
                     third = fmaxf(third, lo);
                 }
-                amb |= lo >= best - thr0;
+                if constexpr (wrap) {
+                    // a group whose runner-up came near gives up its third as well: there is no second look later
+                    const bool near_best = lo >= best - thr0;
+                    if (__any_sync(kAll, near_best)) {
+                        load_scores(tbase + col, bm, 32 * g, v);
+                        float g3 = -INFINITY;
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const float x = tag_score(v[i], i);   // (the tags make the 32 values distinct)
+                            g3 = fmaxf(g3, x == hi || x == lo ? -INFINITY : x);
+                        }
+                        if (near_best) third = fmaxf(third, g3);
+                    }
+                } else {
+                    amb |= lo >= best - thr0;
+                }
                 if constexpr (!wrap) {
                     // for the keys that do need a second look: the groups whose maximum came within the threshold
                     // (with a bias the fp32 additions s + bias round by up to 2^-24 |s + bias| each)
@@ -580,10 +599,13 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     if (dflag) {
                         const unsigned int at = atomicAdd(p.counters + 1, 1u);
                         if (at < p.pool_cap) {
-                            p.pool[at] = make_uint4(last_rec, static_cast<uint32_t>(m) | (static_cast<uint32_t>(unbounded || n > 4 ? 255 : n) << 8), c01, c23);
+                            if (unbounded || n > 4) n = 255;
+                            heavy |= n == 255 || n == 0;
+                            p.pool[at] = make_uint4(last_rec, static_cast<uint32_t>(m) | (static_cast<uint32_t>(n) << 8), c01, c23);
                             last_rec = at;
                             doubt |= 1u << m;
                         } else {
+                            heavy = true;
                             doubt |= 0x100u << m;   // no room for the record: the repair kernel scores every code of this codebook
                         }
                     }
@@ -646,7 +668,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             }
         }
         if (doubt != 0 && ok) {
-            const unsigned int at = atomicAdd(p.counters, 1u);   // at most one entry per key: the list holds every key if need be
+            // at most one entry per key: the two lists together hold every key if need be
+            const unsigned int at = heavy ? p.pool_cap - 1u - atomicAdd(p.counters + 2, 1u) : atomicAdd(p.counters, 1u);
             const unsigned long long lin = static_cast<unsigned long long>(static_cast<int64_t>(u) * p.L + j);
             p.work[at] = make_uint4(static_cast<uint32_t>(lin), static_cast<uint32_t>(lin >> 32), last_rec, doubt);
         }
@@ -668,98 +691,144 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
 
 
 // ------------------------------------------------------------------------------------------------
-// Exact settlement of the doubtful keys.  One warp per list entry: it follows the key through the
+// Exact settlement of the doubtful keys.  A list entry is followed through the
 // codebooks with the defining arithmetic - residual r_0 = k, r_{m+1} = r_m - C_m[code_m] (fp32
-// subtraction) - and settles every doubtful codebook: each score is ONE fused-multiply-add chain over
+// subtraction) - up to its last doubtful codebook: each score is ONE fused-multiply-add chain over
 // d = 0..D-1 starting from +0 (+ bias), ties go to the lowest code.  With a candidate record, one lane
 // per candidate runs the chain; without one (too many candidates, no room for the record, or a code of
-// an earlier codebook has changed and with it the residual) lane l scores the codes l, l + 32, ... of
-// the whole codebook.  The residual is broadcast from shared memory.
-template <typename KT, int D>
-__global__ void __launch_bounds__(kAtRepairWarps * 32)
-assign_repair_kernel(AtParams p)
+// an earlier codebook has changed and with it the residual) the lanes score the whole codebook.
+// Bound by the latency of dependent loads: list entry -> record -> rows.  So the key, its codes and its records are fetched
+// together, then all codebook rows that the residual needs and the first candidates' rows together, into shared memory.
+// A whole codebook (512 KB at K = 1024, D = 128) takes one warp tens of microseconds, so four warps share it: the scan puts
+// such keys on a list of their own, and a warp that changes a code leaves the key's later codebooks to its CTA.
+// (us; 32 heads, D 128; before: one warp per key throughout, rows fetched as they were needed)
+//   32768 bf16 keys, M4 K256: 108 -> 58;  2 x 16384, M4 K512: 300 -> 115;  5001 half keys, M1 K1024: 110 -> 43
+// TEAM: warps that share an entry (1 or kAtRepairWarps); each keeps its own copy of everything but the codebook scan.
+// TEAM = 1 returns the codebooks (bit m) left to the CTA.
+template <int D>
+struct AtRepairBuf {
+    float r[D];                    // residual
+    float row[kAtMaxM][D];         // C_m[code_m] as the scan left the codes
+    float cand[4][D + 4];          // candidate rows (padded: four lanes read four rows)
+    uint4 rec[kAtMaxM];
+};
+
+__device__ __forceinline__ void at_copy16(const float *dst, const float *src)
 {
-    __shared__ __align__(16) float s_r[kAtRepairWarps][D];
-    __shared__ uint4 s_rec[kAtRepairWarps][kAtMaxM];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned int count = p.counters[0];
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+template <typename KT, int D, int TEAM>
+__device__ __forceinline__ uint32_t settle_key(const AtParams &p, const uint4 ent, AtRepairBuf<D> &s, float2 *team_best)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int PER = D / 32;    // residual elements a lane keeps up to date
+    const int lane = threadIdx.x & 31, tw = TEAM > 1 ? threadIdx.x >> 5 : 0;
     const int M = p.M, K = p.K;
-    float *r = s_r[warp];
-    constexpr int PER = D / 32;   // residual elements a lane keeps up to date
-    for (unsigned int e = blockIdx.x * kAtRepairWarps + warp; e < count; e += gridDim.x * kAtRepairWarps) {
-        const uint4 ent = p.work[e];
-        const uint32_t doubt = ent.w & 0xffu, brute = (ent.w >> 8) & 0xffu;
-        const int64_t lin = static_cast<int64_t>((static_cast<unsigned long long>(ent.y) << 32) | ent.x);
-        const int64_t u = lin / p.L, j = lin % p.L;
-        const int b = static_cast<int>(u / p.Hkv), h = static_cast<int>(u % p.Hkv);
-        const KT *krow = static_cast<const KT *>(p.k) + b * p.k_sb + h * p.k_sh + j * p.k_sl;
-        const float *cbh = p.cb + static_cast<int64_t>(h) * M * K * D;
-        __syncwarp();
-        // the key's records, newest first, into a table indexed by codebook
-        if (lane == 0) {
-            uint32_t at = ent.z;
-            for (int guard = 0; guard < kAtMaxM && at != 0xffffffffu && at < p.pool_cap; ++guard) {
-                const uint4 rec = p.pool[at];
-                s_rec[warp][rec.y & 0xffu & (kAtMaxM - 1)] = rec;
-                at = rec.x;
-            }
+    const uint32_t doubt = ent.w & 0xffu, brute = (ent.w >> 8) & 0xffu;
+    const int64_t lin = static_cast<int64_t>((static_cast<unsigned long long>(ent.y) << 32) | ent.x);
+    const int64_t u = lin / p.L, j = lin % p.L;
+    const int b = static_cast<int>(u / p.Hkv), h = static_cast<int>(u % p.Hkv);
+    const KT *krow = static_cast<const KT *>(p.k) + b * p.k_sb + h * p.k_sh + j * p.k_sl;
+    const float *cbh = p.cb + static_cast<int64_t>(h) * M * K * D;
+    const int64_t cbase = b * p.c_sb + h * p.c_sh + j * p.c_sl;
+    __syncwarp();                  // the previous entry's reads of the buffers
+    const int my_code = lane < M ? load_code(p.codes, p.code_dtype, cbase + lane) : 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) s.r[lane + 32 * i] = to_f32(krow[lane + 32 * i]);
+    // the key's records, newest first, into a table indexed by codebook
+    if (lane == 0) {
+        uint32_t at = ent.z;
+        for (int guard = 0; guard < kAtMaxM && at != 0xffffffffu && at < p.pool_cap; ++guard) {
+            const uint4 rec = p.pool[at];
+            s.rec[rec.y & 0xffu & (kAtMaxM - 1)] = rec;
+            at = rec.x;
         }
+    }
+    if (TEAM > 1) __syncthreads();   // every warp has read the codes before one of them may rewrite them
+    else __syncwarp();
+    const int last = 31 - __clz(static_cast<int>(doubt | brute));   // (an entry has at least one doubtful codebook)
+    auto copy_row = [&](float *dst, int m, int code) {
+        if (lane < D / 4) at_copy16(dst + 4 * lane, cbh + (static_cast<int64_t>(m) * K + code) * D + 4 * lane);
+    };
+    auto candidate = [](const uint4 &rec, int i) { return static_cast<int>(((i < 2 ? rec.z : rec.w) >> (16 * (i & 1))) & 0xffffu); };
+    auto candidates = [&](int m) { return ((doubt >> m) & 1u) ? static_cast<int>((s.rec[m].y >> 8) & 0xffu) : 0; };
+    auto copy_candidates = [&](int m, int n) {
+        const uint4 rec = s.rec[m];
+        for (int i = 0; i < n; ++i) copy_row(s.cand[i], m, min(candidate(rec, i), K - 1));
+    };
+    for (int m = 0; m < last; ++m) copy_row(s.row[m], m, __shfl_sync(kAll, my_code, m));
+    const int first = doubt ? __ffs(doubt) - 1 : -1;   // its candidates travel with the rows
+    if (first >= 0 && candidates(first) <= 4) copy_candidates(first, candidates(first));
+    bool changed = false;
+    for (int m = 0; m < M && (changed || m <= last); ++m) {
+        const int old = __shfl_sync(kAll, my_code, m);
+        int code = old;
+        const bool dm = (doubt >> m) & 1u;
+        const int ncand = candidates(m);
+        const bool all = changed || ((brute >> m) & 1u) || (dm && (ncand > 4 || ncand == 0));
+        if (all || dm) {
+            const float *cm = cbh + static_cast<int64_t>(m) * K * D;
+            const float *bm = p.bias ? p.bias + (static_cast<int64_t>(h) * M + m) * K : nullptr;
+            float bv = -INFINITY;
+            int bi = 0x7fffffff;
+            if (all) {
+                bi = 0;                                     // no score above -inf (NaN scores): the first code, as in the exact kernel
+                constexpr int R = 2;                        // codes per lane at a time, eight 16-byte loads of each in flight
+                for (int c0 = 32 * R * tw; c0 < K; c0 += 32 * R * TEAM) {
+                    float acc[R];
+                    const float *row[R];
 #pragma unroll
-        for (int i = 0; i < PER; ++i) r[lane + 32 * i] = to_f32(krow[lane + 32 * i]);
-        __syncwarp();
-        const int64_t cbase = b * p.c_sb + h * p.c_sh + j * p.c_sl;
-        bool changed = false;
-        for (int m = 0; m < M; ++m) {
-            int code = load_code(p.codes, p.code_dtype, cbase + m);
-            const bool dm = (doubt >> m) & 1u;
-            const uint4 rec = dm ? s_rec[warp][m] : make_uint4(0, 0, 0, 0);
-            const int ncand = static_cast<int>((rec.y >> 8) & 0xffu);
-            const bool all = changed || ((brute >> m) & 1u) || (dm && (ncand > 4 || ncand == 0));
-            if (all || dm) {
-                const float *cm = cbh + static_cast<int64_t>(m) * K * D;
-                const float *bm = p.bias ? p.bias + (static_cast<int64_t>(h) * M + m) * K : nullptr;
-                float bv = -INFINITY;
-                int bi = 0x7fffffff;
-                if (all) {
-                    bi = 0;                                     // no score above -inf (NaN scores): the first code, as in the exact kernel
-                    for (int c0 = 0; c0 < K; c0 += 128) {       // four codes per lane at a time: four independent chains
-                        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                        const float *row[4];
+                    for (int t = 0; t < R; ++t) {
+                        acc[t] = 0.f;
+                        row[t] = cm + static_cast<int64_t>(min(c0 + lane + 32 * t, K - 1)) * D;
+                    }
+#pragma unroll 1
+                    for (int d0 = 0; d0 < D; d0 += 32) {
+                        float4 c4[R][8];
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) row[t] = cm + static_cast<int64_t>(min(c0 + lane + 32 * t, K - 1)) * D;
-#pragma unroll 4
-                        for (int d = 0; d < D; d += 4) {
-                            const float4 r4 = *reinterpret_cast<const float4 *>(r + d);
+                        for (int t = 0; t < R; ++t)
 #pragma unroll
-                            for (int t = 0; t < 4; ++t) {
-                                const float4 c4 = __ldg(reinterpret_cast<const float4 *>(row[t] + d));
-                                acc[t] = __fmaf_rn(r4.x, c4.x, acc[t]);
-                                acc[t] = __fmaf_rn(r4.y, c4.y, acc[t]);
-                                acc[t] = __fmaf_rn(r4.z, c4.z, acc[t]);
-                                acc[t] = __fmaf_rn(r4.w, c4.w, acc[t]);
-                            }
-                        }
+                            for (int e = 0; e < 8; ++e) c4[t][e] = __ldg(reinterpret_cast<const float4 *>(row[t] + d0 + 4 * e));
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) {
-                            const int c = c0 + lane + 32 * t;
-                            if (c < K) {
-                                const float sc = bm ? __fadd_rn(acc[t], __ldg(bm + c)) : acc[t];
-                                if (sc > bv) {      // codes come in increasing order: the first maximum stays
-                                    bv = sc;
-                                    bi = c;
-                                }
+                        for (int e = 0; e < 8; ++e) {
+                            const float4 r4 = *reinterpret_cast<const float4 *>(s.r + d0 + 4 * e);
+#pragma unroll
+                            for (int t = 0; t < R; ++t) {
+                                acc[t] = __fmaf_rn(r4.x, c4[t][e].x, acc[t]);
+                                acc[t] = __fmaf_rn(r4.y, c4[t][e].y, acc[t]);
+                                acc[t] = __fmaf_rn(r4.z, c4[t][e].z, acc[t]);
+                                acc[t] = __fmaf_rn(r4.w, c4[t][e].w, acc[t]);
                             }
                         }
                     }
-                } else if (lane < ncand) {
-                    const int c = static_cast<int>(((lane < 2 ? rec.z : rec.w) >> (16 * (lane & 1))) & 0xffffu);
+#pragma unroll
+                    for (int t = 0; t < R; ++t) {
+                        const int c = c0 + lane + 32 * t;
+                        if (c < K) {
+                            const float sc = bm ? __fadd_rn(acc[t], __ldg(bm + c)) : acc[t];
+                            if (sc > bv) {      // codes come in increasing order: the first maximum stays
+                                bv = sc;
+                                bi = c;
+                            }
+                        }
+                    }
+                }
+            } else {
+                if (m != first) {
+                    __syncwarp();
+                    copy_candidates(m, ncand);
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                __syncwarp();
+                if (lane < ncand) {
+                    const int c = candidate(s.rec[m], lane);
                     if (c < K) {
-                        const float *crow = cm + static_cast<int64_t>(c) * D;
                         float acc = 0.f;
 #pragma unroll 8
                         for (int d = 0; d < D; d += 4) {
-                            const float4 r4 = *reinterpret_cast<const float4 *>(r + d);
-                            const float4 c4 = __ldg(reinterpret_cast<const float4 *>(crow + d));
+                            const float4 r4 = *reinterpret_cast<const float4 *>(s.r + d);
+                            const float4 c4 = *reinterpret_cast<const float4 *>(s.cand[lane] + d);
                             acc = __fmaf_rn(r4.x, c4.x, acc);
                             acc = __fmaf_rn(r4.y, c4.y, acc);
                             acc = __fmaf_rn(r4.z, c4.z, acc);
@@ -769,30 +838,90 @@ assign_repair_kernel(AtParams p)
                         bi = c;
                     }
                 }
+            }
 #pragma unroll
-                for (int off = 16; off >= 1; off >>= 1) {
-                    const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-                    if (ov > bv || (ov == bv && oi < bi)) {
-                        bv = ov;
+            for (int off = 16; off >= 1; off >>= 1) {
+                const float ov = __shfl_xor_sync(kAll, bv, off);
+                const int oi = __shfl_xor_sync(kAll, bi, off);
+                if (ov > bv || (ov == bv && oi < bi)) {
+                    bv = ov;
+                    bi = oi;
+                }
+            }
+            if (TEAM > 1 && all) {   // (`all` is the same in every warp of the team: so is all that it is formed from)
+                __syncthreads();
+                if (lane == 0) team_best[tw] = make_float2(bv, __int_as_float(bi));
+                __syncthreads();
+#pragma unroll
+                for (int t = 0; t < TEAM; ++t) {
+                    const float2 o = team_best[t];
+                    const int oi = __float_as_int(o.y);
+                    if (o.x > bv || (o.x == bv && oi < bi)) {
+                        bv = o.x;
                         bi = oi;
                     }
                 }
-                if (bi != code && bi != 0x7fffffff) {
-                    changed = true;
-                    code = bi;
-                    if (lane == 0) store_code(p.codes, p.code_dtype, cbase + m, code);
+            }
+            if (bi != code && bi != 0x7fffffff) {
+                changed = true;
+                code = bi;
+                if (lane == 0 && tw == 0) store_code(p.codes, p.code_dtype, cbase + m, code);
+                if (TEAM == 1 && m + 1 < M) {
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    return ((1u << M) - 1u) & ~((2u << m) - 1u);
                 }
             }
-            if (m + 1 < M) {
-                const float *crow = cbh + (static_cast<int64_t>(m) * K + code) * D;
-                __syncwarp();
+        }
+        if (m + 1 < M && (changed || m < last)) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+            const bool have = code == old && m < last;       // the row that was fetched ahead
+            const float *crow = cbh + (static_cast<int64_t>(m) * K + code) * D;
 #pragma unroll
-                for (int i = 0; i < PER; ++i) r[lane + 32 * i] = __fsub_rn(r[lane + 32 * i], __ldg(crow + lane + 32 * i));
-                __syncwarp();
+            for (int i = 0; i < PER; ++i) {
+                const float c = have ? s.row[m][lane + 32 * i] : __ldg(crow + lane + 32 * i);
+                s.r[lane + 32 * i] = __fsub_rn(s.r[lane + 32 * i], c);
             }
+            __syncwarp();
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return 0u;
+}
+
+template <typename KT, int D>
+__global__ void __launch_bounds__(kAtRepairWarps * 32)
+assign_repair_kernel(AtParams p)
+{
+    __shared__ __align__(16) AtRepairBuf<D> s_buf[kAtRepairWarps];
+    __shared__ float2 s_team[kAtRepairWarps];
+    __shared__ uint4 s_left[kAtLeft];          // keys whose later codebooks are left to the CTA
+    __shared__ unsigned int s_nleft;
+    const int warp = threadIdx.x >> 5;
+    const unsigned int count = p.counters[0], heavy = p.counters[2];
+    if (threadIdx.x == 0) s_nleft = 0u;
+    __syncthreads();
+    // the long ones first: they are spread over all CTAs
+    for (unsigned int e = blockIdx.x; e < heavy; e += gridDim.x) settle_key<KT, D, kAtRepairWarps>(p, p.work[p.pool_cap - 1u - e], s_buf[warp], s_team);
+    for (unsigned int e = blockIdx.x * kAtRepairWarps + warp; e < count; e += gridDim.x * kAtRepairWarps) {
+        uint4 ent = p.work[e];
+        const uint32_t left = settle_key<KT, D, 1>(p, ent, s_buf[warp], nullptr);
+        if (left == 0u) continue;
+        // every code up to the changed one is settled; the codebooks after it are scored in full
+        ent.z = 0xffffffffu;
+        ent.w = left << 8;
+        unsigned int at = 0;
+        if ((threadIdx.x & 31) == 0) at = atomicAdd(&s_nleft, 1u);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (at < kAtLeft) {
+            if ((threadIdx.x & 31) == 0) s_left[at] = ent;
+        } else {
+            while (ent.w != 0u) ent.w = settle_key<KT, D, 1>(p, ent, s_buf[warp], nullptr) << 8;   // no room: one changed code at a time
+        }
+    }
+    __syncthreads();
+    const unsigned int nleft = s_nleft < kAtLeft ? s_nleft : kAtLeft;
+    for (unsigned int e = 0; e < nleft; ++e) settle_key<KT, D, kAtRepairWarps>(p, s_left[e], s_buf[warp], s_team);
 }
 
 template <typename KT, int D, int NS, int CH, bool WRAP = false>
