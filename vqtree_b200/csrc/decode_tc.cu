@@ -21,6 +21,8 @@
 // The global list of tiles is split evenly over the CTAs (a range may start or end inside a unit);
 // a CTA writes one partial (numerator, maximum, denominator) per unit it touched and the last CTA
 // of a unit (atomic ticket) merges them - the same workspace protocol as the SIMT bulk kernel.
+// The launch overlaps its neighbours in the stream (see launch_overlapped): a generated token of one 7B-shaped sequence, 23.4 -> 21.1 us
+// with its rotate-and-append launch, eight grouped-query sequences 38.5 -> 35.1 us.
 // Every wait is bounded; a failed wait raises the status word and the CTA leaves; TMEM is freed.
 #include "decode_common.cuh"
 #include "prefill_tc_common.cuh"
@@ -186,7 +188,13 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
                 dt_bulk_copy(cnt_s + st * kDtRows, p.cnt + static_cast<int64_t>(ue) * p.MK + it.row0, kDtRows * 4, &full[st]);
         }
     };
-    if (producer) produce(min(n_items, NS));   // the ring is empty: no wait inside
+    // The launch may overlap the kernel before it (a generated token: rotate-and-append) and lets the one after it start its
+    // own prologue: barriers and tensor memory are set up meanwhile, global memory is touched only behind the wait.
+    grid_dependency_launch();
+    if (producer) {
+        grid_dependency_wait();
+        produce(min(n_items, NS));   // the ring is empty: no wait inside
+    }
     if (warp == 4) {
         __syncwarp();
         tmem_alloc(&s_tmem, 64);
@@ -195,6 +203,7 @@ decode_tc_kernel(const __grid_constant__ CUtensorMap tm_k1, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();        // every thread: outputs, partials and tickets
     const uint32_t tmem = s_tmem;  // columns: S^T buffers at 0 and 16, O^T buffers at 32 and 48 (the unit segments alternate)
 
     if (warp == 5) {
@@ -663,8 +672,7 @@ int launch_decode_tc(const VqDecodeArgs *a, const DecodeParams &p, cudaStream_t 
             if (dev >= 0 && dev < 64) opted[dev] = true;
         }
     }
-    decode_tc_kernel<<<bp.num_ctas, kDtThreads, kDtSmem, s>>>(mk1, mk3, mv, mcb, mvs, mq1, mq2, bp);
-    return launch_status();
+    return launch_overlapped(decode_tc_kernel, dim3(static_cast<unsigned>(bp.num_ctas)), dim3(kDtThreads), kDtSmem, s, mk1, mk3, mv, mcb, mvs, mq1, mq2, bp);
 }
 
 }  // namespace vq

@@ -178,6 +178,8 @@ __global__ void __launch_bounds__(256) rope_multi_kernel(const RopeMultiParams p
 {
     constexpr int N = RopeVec<T>::kN;
     const int half = p.D / 2, tpr = half / N;
+    grid_dependency_launch();   // the attention of a generated token follows: its CTAs come up meanwhile
+    grid_dependency_wait();
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < p.total;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         int j = 0;
@@ -333,13 +335,18 @@ static int rope_add_job(RopeMultiParams &p, const VqTensorDesc *x, const VqTenso
     return VQ_OK;
 }
 
-static int rope_multi_launch(const RopeMultiParams &p, int dtype, cudaStream_t s)
+static int rope_multi_launch(const RopeMultiParams &p, int dtype, cudaStream_t s, bool overlapped = false)
 {
     if (p.total == 0) return VQ_OK;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return VQ_EDEVICE;
     const int64_t want = (p.total + 255) / 256;
     const unsigned grid = static_cast<unsigned>(want < static_cast<int64_t>(sms) * 16 ? want : static_cast<int64_t>(sms) * 16);
+    if (overlapped) {
+        if (dtype == VQ_F32) return launch_overlapped(rope_multi_kernel<float>, dim3(grid), dim3(256), 0, s, p);
+        if (dtype == VQ_F16) return launch_overlapped(rope_multi_kernel<__half>, dim3(grid), dim3(256), 0, s, p);
+        return launch_overlapped(rope_multi_kernel<__nv_bfloat16>, dim3(grid), dim3(256), 0, s, p);
+    }
     if (dtype == VQ_F32) rope_multi_kernel<float><<<grid, 256, 0, s>>>(p);
     else if (dtype == VQ_F16) rope_multi_kernel<__half><<<grid, 256, 0, s>>>(p);
     else rope_multi_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(p);
@@ -471,5 +478,5 @@ extern "C" int vqattn_decode_append(const VqTensorDesc *q, const VqTensorDesc *k
     if ((st = rope_add_job(p, q, q1, q2, nullptr, 0, vec)) != VQ_OK) return st;
     if ((st = rope_add_job(p, k, k1_win, nullptr, k3_win, row, vec)) != VQ_OK) return st;
     if ((st = rope_add_job(p, v, nullptr, nullptr, v_win, row, vec)) != VQ_OK) return st;
-    return rope_multi_launch(p, q->dtype, static_cast<cudaStream_t>(stream));
+    return rope_multi_launch(p, q->dtype, static_cast<cudaStream_t>(stream), true);
 }

@@ -53,6 +53,28 @@ inline int launch_status()
     return cudaGetLastError() == cudaSuccess ? VQ_OK : VQ_ELAUNCH;
 }
 
+// Launch that may begin before the previous kernel of the stream has ended (programmatic dependent launch).  The kernel calls
+// grid_dependency_wait() in every thread before it touches memory that another kernel reads or writes: from there on everything
+// earlier in the stream is complete and visible, as after an ordinary launch.
+template <typename... KArgs, typename... Args>
+inline int launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Args &&>(args)...) == cudaSuccess ? VQ_OK : VQ_ELAUNCH;
+}
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// lets the next kernel of the stream start its prologue (if it was launched with launch_overlapped)
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 x) { return __bfloat162float(x); }
 __device__ __forceinline__ float to_f32(__half x) { return __half2float(x); }
