@@ -134,7 +134,8 @@ int vqattn_build_aggregates(const VqTensorDesc *codes, const VqTensorDesc *v, in
  * The same with a caller workspace of vqattn_aggregates_workspace_bytes(B, Hkv, NB, M, K) bytes (device memory,
  * 16-byte aligned; contents need not be preserved between calls): the keys of every 128-key block are sorted by
  * code once, so that the kernel that forms the sums reads each row's keys instead of scanning the block's codes.
- * Same results, bit for bit.  Used for bf16 values and sums with D = 64 or 128 and K a multiple of 8 up to 4096;
+ * Same results, bit for bit.  Used for values and sums of one type with D = 64 or 128 and K a multiple of 8 up to 4096
+ * (half, fp32: K up to 256 or a multiple of it);
  * other inputs, a NULL workspace or one that is too small take the path of vqattn_build_aggregates.
  * A code outside [0, K) is left out and reported through status_word (VQ_WORD_BAD_CODE; may be NULL).
  */
@@ -319,6 +320,15 @@ int vqattn_decode_step(const VqDecodeStepArgs *args, void *stream);
  */
 int vqattn_cache_advance(const VqTensorDesc *codes, const VqTensorDesc *v_new, int32_t K, VqTensorDesc *cnt,
                          VqTensorDesc *vsum_f32, VqTensorDesc *vsum_act_or_null, int32_t *status_word, void *stream);
+
+/*
+ * What a prefill leaves in a decode cache (ops/attn_vq.py:89-127 update_prefill), in one launch: the last n rows of the rotated
+ * keys, raw keys and values [B,Hkv,n,D] (strided, contiguous last dim) become rows [0, n) of the window buffers [B,Hkv,cap,D]
+ * (dense, cap >= n), rows [n, cap) are zeroed; vsum_act NULL or [B,Hkv,MK,D] in the 16-bit activation dtype: vsum_f32 rounded.
+ */
+int vqattn_store_window(const VqTensorDesc *k1, const VqTensorDesc *k3, const VqTensorDesc *v, VqTensorDesc *k1_win,
+                        VqTensorDesc *k3_win, VqTensorDesc *v_win, const VqTensorDesc *vsum_f32, VqTensorDesc *vsum_act_or_null,
+                        void *stream);
 
 #ifdef __cplusplus
 }

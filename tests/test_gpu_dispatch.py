@@ -122,3 +122,18 @@ def test_prefill_fp32_equals_the_row_kernel(api, L, W, D, Hq, Hkv, M, K, rerope)
     assert torch.equal(torch.isinf(got), torch.isinf(want))
     ok = ~torch.isinf(want)
     assert (got[ok] - want[ok]).abs().max() < 2e-5 and (lse - lse_w).abs().max() < 2e-5
+
+
+# the window a prefill leaves behind: whole vectors, and single elements where rows or addresses are no multiples of 16 bytes
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("n,cap,D,pad", [(1, 3, 64, 0), (130, 512, 128, 0), (57, 57, 128, 3), (9, 20, 40, 1)])
+def test_store_window_copies_and_zeroes(api, dtype, n, cap, D, pad):
+    g = _gen(n)
+    src = [_rn(g, 2, n + 5, 3, D + pad).to(dtype).transpose(1, 2)[:, :, 5:, pad:] for _ in range(3)]
+    win = [torch.full((2, 3, cap, D), 7.0, dtype=dtype, device="cuda") for _ in range(3)]
+    vs = _rn(g, 2, 3, 8, D) * 1e5
+    act = None if dtype == torch.float32 else torch.empty(vs.shape, dtype=dtype, device="cuda")
+    api.store_window(*src, *win, vs if act is not None else None, act)
+    for s, w in zip(src, win):
+        assert torch.equal(w[:, :, :n], s) and not w[:, :, n:].any()
+    assert act is None or torch.equal(act, vs.to(dtype))

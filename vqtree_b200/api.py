@@ -436,6 +436,15 @@ def cache_advance(codes, v_new, K: int, cnt, vsum_f32, vsum_act=None):
                                        device_status_word(dev).data_ptr(), stream_ptr(dev)), "vqattn_cache_advance")
 
 
+def store_window(k1, k3, v, k1_win, k3_win, v_win, vsum_f32=None, vsum_act=None) -> None:
+    """The window a prefill leaves behind, in one launch: k1, k3, v [B,Hkv,n,D] -> rows [0, n) of the buffers [B,Hkv,cap,D], zeros
+    behind them; vsum_act (optional): vsum_f32 rounded to its dtype."""
+    dev = _require_cuda(k1, k3, v, k1_win, k3_win, v_win, vsum_f32, vsum_act)
+    with torch.cuda.device(dev):
+        check(lib.vqattn_store_window(desc(k1), desc(k3), desc(v), desc(k1_win), desc(k3_win), desc(v_win), desc(vsum_f32), desc(vsum_act),
+                                      stream_ptr(dev)), "vqattn_store_window")
+
+
 # ---------------------------------------------------------------------------------------------
 # Host-buffer entry points: CPU tensors in, CPU tensor out, copies included.
 

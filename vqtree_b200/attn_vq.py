@@ -175,13 +175,25 @@ class VectorQuantizedReRoPECache(_HFCache):
         B, Hkv, n_local, D = local_key.shape
         dev, dt = local_key.device, local_key.dtype
         cap = 2 * (self.window_length + 2 * BLOCK_SIZE)     # window slides through the buffer; see _make_room
-        bufs = [torch.zeros(B, Hkv, cap, D, dtype=dt, device=dev) for _ in range(3)]
-        for buf, src in zip(bufs, (local_key, raw, local_value)):
-            buf[:, :, :n_local] = src
+        srcs = (local_key, raw, local_value)
         vs32 = cumulated_value.float().contiguous()
+        vsum = None
+        if (dt in (torch.float16, torch.bfloat16, torch.float32) and n_local > 0 and vs32.dim() == 4 and vs32.numel() % 4 == 0
+                and all(t.is_cuda and t.device == dev and t.dtype == dt and t.shape == local_key.shape and t.stride(-1) == 1
+                        and not (t.requires_grad and torch.is_grad_enabled()) for t in srcs)
+                and vs32.device == dev and vs32.data_ptr() % 16 == 0 and not (vs32.requires_grad and torch.is_grad_enabled())):
+            bufs = [torch.empty(B, Hkv, cap, D, dtype=dt, device=dev) for _ in range(3)]
+            if dt != torch.float32:
+                vsum = torch.empty(vs32.shape, dtype=dt, device=dev)
+            api.store_window(*srcs, *bufs, vs32 if vsum is not None else None, vsum)
+        else:                                               # host tensors, mixed types, tracked gradients
+            bufs = [torch.zeros(B, Hkv, cap, D, dtype=dt, device=dev) for _ in range(3)]
+            for buf, src in zip(bufs, srcs):
+                buf[:, :, :n_local] = src
+            vsum = None if dt == torch.float32 else vs32.to(dt)
         self.states[layer_idx] = dict(
             n=num_tokens, bd=num_tokens - n_local, start=0, cap=cap, win_k1=bufs[0], win_k3=bufs[1], win_v=bufs[2],
-            cnt=cumulated_key.float().contiguous(), vsum32=vs32, vsum=None if dt == torch.float32 else vs32.to(dt),
+            cnt=cumulated_key.float().contiguous(), vsum32=vs32, vsum=vsum,
             q1=None, q2=None, call=None)
         if layer_idx == 0:
             self.seen_tokens += num_tokens

@@ -26,7 +26,7 @@ OBJDIR = PKG / "build"
 LIB = LIBDIR / "libvqattn.so"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-SOURCES = ["api.cu", "assign.cu", "assign_tc.cu", "aggregate.cu", "aggregate_reg.cu", "prefill_simt.cu", "prefill_f32.cu", "prefill_tc4.cu", "rope.cu", "decode.cu", "decode_bulk.cu", "decode_tc.cu"]
+SOURCES = ["api.cu", "assign.cu", "assign_tc.cu", "aggregate.cu", "aggregate_reg.cu", "prefill_simt.cu", "prefill_f32.cu", "prefill_tc4.cu", "rope.cu", "decode.cu", "decode_bulk.cu", "decode_tc.cu", "window.cu"]
 
 
 def nvcc_path() -> str:

@@ -36,7 +36,7 @@ EXPORTS = (
     "vqattn_cache_advance", "vqattn_decode_static_capacity", "vqattn_decode_static",
     "vqattn_assign_workspace_bytes", "vqattn_assign_codes_ws", "vqattn_rope",
     "vqattn_status_from_word", "vqattn_set_wait_limit_cycles", "vqattn_wait_selftest", "vqattn_rope_qk",
-    "vqattn_decode_append", "vqattn_decode_step",
+    "vqattn_decode_append", "vqattn_decode_step", "vqattn_store_window",
 )
 
 
@@ -114,6 +114,7 @@ def _load() -> ctypes.CDLL:
     lib.vqattn_decode_static_capacity.restype = ctypes.c_size_t
     lib.vqattn_cache_advance.argtypes = [P(VqTensorDesc), P(VqTensorDesc), ctypes.c_int32, P(VqTensorDesc),
                                          P(VqTensorDesc), P(VqTensorDesc), ctypes.c_void_p, ctypes.c_void_p]
+    lib.vqattn_store_window.argtypes = [P(VqTensorDesc)] * 8 + [ctypes.c_void_p]
     lib.vqattn_rope_qk.argtypes = [P(VqTensorDesc), P(VqTensorDesc), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                    ctypes.c_int64, ctypes.c_int64, P(VqTensorDesc), P(VqTensorDesc), P(VqTensorDesc),
                                    ctypes.c_void_p, ctypes.c_void_p]
@@ -156,17 +157,18 @@ def desc(t: torch.Tensor | None, d: VqTensorDesc | None = None) -> VqTensorDesc:
     if t is None:
         d.ptr = None
         return d
-    if t.dtype not in _DTYPES:
+    dtype = _DTYPES.get(t.dtype)
+    if dtype is None:
         raise TypeError(f"unsupported dtype {t.dtype}")
-    if t.dim() > MAX_DIMS:
+    n = t.dim()
+    if n > MAX_DIMS:
         raise ValueError("too many dimensions")
     d.ptr = t.data_ptr()
-    d.dtype = _DTYPES[t.dtype]
-    d.ndim = t.dim()
-    for i in range(t.dim()):
-        d.shape[i] = t.shape[i]
-        d.stride[i] = t.stride(i)
-    d.device = t.device.index if t.is_cuda else -1
+    d.dtype = dtype
+    d.ndim = n
+    d.shape[:n] = t.shape       # one assignment per array: a layer's call fills some thirty descriptors
+    d.stride[:n] = t.stride()
+    d.device = t.get_device()   # -1: host memory
     return d
 
 
