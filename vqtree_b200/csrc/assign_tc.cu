@@ -182,16 +182,17 @@ __device__ __forceinline__ void load_scores(uint32_t taddr, const float *bm, int
     }
 }
 
-// four residual columns as bf16 hi and lo terms, 8 bytes each, at byte `off` of the two operand tiles
+// four residual columns as bf16 hi and lo terms, 8 bytes each, at byte `off` of the two operand tiles (packed conversions:
+// single ones run on the special-function unit, a quarter of the rate)
 __device__ __forceinline__ void store_terms(uint8_t *a_rh, uint8_t *a_rl, uint32_t off, const float (&x)[4])
 {
     uint32_t wh[2], wl[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-        const __nv_bfloat16 h0 = __float2bfloat16_rn(x[2 * e]), h1 = __float2bfloat16_rn(x[2 * e + 1]);
-        __nv_bfloat162 hv = __halves2bfloat162(h0, h1);
-        wh[e] = *reinterpret_cast<uint32_t *>(&hv);
-        wl[e] = pack_bf16(x[2 * e] - __bfloat162float(h0), x[2 * e + 1] - __bfloat162float(h1));
+        wh[e] = pack_bf16(x[2 * e], x[2 * e + 1]);
+        float l0, l1;   // x - hi
+        ffma2(l0, l1, __uint_as_float(wh[e] << 16), __uint_as_float(wh[e] & 0xffff0000u), -1.f, -1.f, x[2 * e], x[2 * e + 1]);
+        wl[e] = pack_bf16(l0, l1);
     }
     *reinterpret_cast<uint2 *>(a_rh + off) = make_uint2(wh[0], wh[1]);
     *reinterpret_cast<uint2 *>(a_rl + off) = make_uint2(wl[0], wl[1]);
@@ -642,10 +643,11 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                                           __uint_as_float(vh.y & 0xffff0000u)};
                             if (kConv || m > 0) {
                                 const uint2 vl = *reinterpret_cast<const uint2 *>(a_rl + off);
-                                x[0] += __uint_as_float(vl.x << 16); x[1] += __uint_as_float(vl.x & 0xffff0000u);
-                                x[2] += __uint_as_float(vl.y << 16); x[3] += __uint_as_float(vl.y & 0xffff0000u);
+                                fadd2(x[0], x[1], x[0], x[1], __uint_as_float(vl.x << 16), __uint_as_float(vl.x & 0xffff0000u));
+                                fadd2(x[2], x[3], x[2], x[3], __uint_as_float(vl.y << 16), __uint_as_float(vl.y & 0xffff0000u));
                             }
-                            x[0] -= crow4[i].x; x[1] -= crow4[i].y; x[2] -= crow4[i].z; x[3] -= crow4[i].w;
+                            ffma2(x[0], x[1], crow4[i].x, crow4[i].y, -1.f, -1.f, x[0], x[1]);
+                            ffma2(x[2], x[3], crow4[i].z, crow4[i].w, -1.f, -1.f, x[2], x[3]);
                             store_terms(a_rh, a_rl, off, x);
                         }
                     }
