@@ -176,9 +176,12 @@ __device__ __forceinline__ void load_scores(uint32_t taddr, const float *bm, int
     tmem_ld32(taddr, r);
     tc_wait_ld();
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        v[i] = __uint_as_float(r[i]);
-        if (bm) v[i] += __ldg(bm + c0 + i);
+    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+    // one branch over all of it: tested per element, the loads and additions are issued predicated off (a seventh of the
+    // kernel's instructions)
+    if (bm != nullptr) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] += __ldg(bm + c0 + i);
     }
 }
 
