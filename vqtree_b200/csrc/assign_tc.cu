@@ -185,9 +185,17 @@ __device__ __forceinline__ void load_scores(uint32_t taddr, const float *bm, int
     }
 }
 
+__device__ __forceinline__ void st_shared8(uint32_t addr, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory"); }
+__device__ __forceinline__ uint2 ld_shared8(uint32_t addr)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
 // four residual columns as bf16 hi and lo terms, 8 bytes each, at byte `off` of the two operand tiles (packed conversions:
 // single ones run on the special-function unit, a quarter of the rate)
-__device__ __forceinline__ void store_terms(uint8_t *a_rh, uint8_t *a_rl, uint32_t off, const float (&x)[4])
+__device__ __forceinline__ void store_terms(uint32_t a_rh, uint32_t a_rl, uint32_t off, const float (&x)[4])   // shared-memory addresses
 {
     uint32_t wh[2], wl[2];
 #pragma unroll
@@ -197,8 +205,8 @@ __device__ __forceinline__ void store_terms(uint8_t *a_rh, uint8_t *a_rl, uint32
         ffma2(l0, l1, __uint_as_float(wh[e] << 16), __uint_as_float(wh[e] & 0xffff0000u), -1.f, -1.f, x[2 * e], x[2 * e + 1]);
         wl[e] = pack_bf16(l0, l1);
     }
-    *reinterpret_cast<uint2 *>(a_rh + off) = make_uint2(wh[0], wh[1]);
-    *reinterpret_cast<uint2 *>(a_rl + off) = make_uint2(wl[0], wl[1]);
+    st_shared8(a_rh + off, wh[0], wh[1]);
+    st_shared8(a_rl + off, wl[0], wl[1]);
 }
 
 // WRAP: a codebook has more chunks than the stream's score region holds and goes through it in rounds.
@@ -360,7 +368,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         const bool valid = j < p.L;
         const uint32_t tbase = tmem + (static_cast<uint32_t>(wq * 32) << 16) + s * C::kRegion;
         const float *cbh = p.cb + static_cast<int64_t>(h) * MK * D;
-        uint8_t *a_rh = smem + s * 2 * C::kATile, *a_rl = a_rh + C::kATile;
+        uint8_t *a_tile = smem + s * 2 * C::kATile;
+        const uint32_t a_rh = smem_u32(a_tile), a_rl = a_rh + C::kATile;
         const int groups = K / 32, g_lo = hf * (groups / 2), g_hi = g_lo + groups / 2;
         float4 *xch = &s_x[s][row];
         float rbound;  // |k| + sum of the largest codeword norms so far: a priori bound of the residual's norm
@@ -406,7 +415,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             float ss = 0.f;
 #pragma unroll 4
             for (int ck = 0; ck < D / 8; ++ck) {
-                const uint4 raw = *reinterpret_cast<const uint4 *>(a_rh + (ck >> 3) * kHalfBytes + row * 128 + (((ck & 7) ^ (row & 7)) << 4));
+                const uint4 raw = *reinterpret_cast<const uint4 *>(a_tile + (ck >> 3) * kHalfBytes + row * 128 + (((ck & 7) ^ (row & 7)) << 4));
                 const __nv_bfloat162 *hp = reinterpret_cast<const __nv_bfloat162 *>(&raw);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -451,18 +460,15 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 top2_32(v, hi, lo);
                 // hi, then lo (<= hi) into the sorted triple (best, second, third); a tie with the best goes to the
                 // earlier group, which holds the lower codes
-                if (hi > best) {
-                    third = second; second = best; sgrp = bgrp; best = hi; bgrp = g;
-                } else if (hi > second) {
-                    third = second; second = hi; sgrp = g;
-                } else {
-                    third = fmaxf(third, hi);
-                }
-                if (lo > second) {
-                    third = second; second = lo; sgrp = g;
-                } else {
-                    third = fmaxf(third, lo);
-                }
+                // (minima, maxima and selects: as branches the lanes of a warp take different ones)
+                const bool new_best = hi > best;
+                const float beaten = fminf(hi, best), s1 = fmaxf(second, beaten);
+                sgrp = new_best ? bgrp : hi > second ? g : sgrp;
+                sgrp = lo > s1 ? g : sgrp;
+                bgrp = new_best ? g : bgrp;
+                third = fmax3(third, fminf(second, beaten), fminf(s1, lo));
+                second = fmaxf(s1, lo);
+                best = fmaxf(best, hi);
                 if constexpr (wrap) {
                     // a group whose runner-up came near gives up its third as well: there is no second look later
                     const bool near_best = lo >= best - thr0;
@@ -641,11 +647,11 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                         for (int i = 0; i < NB; ++i) {
                             const int r = wq * 32 + 16 * hf + (i0 + i) * KPI + sub;
                             const uint32_t off = lane_off + r * 128 + ((chunk ^ (r & 7)) << 4);
-                            const uint2 vh = *reinterpret_cast<const uint2 *>(a_rh + off);
+                            const uint2 vh = ld_shared8(a_rh + off);
                             float x[4] = {__uint_as_float(vh.x << 16), __uint_as_float(vh.x & 0xffff0000u), __uint_as_float(vh.y << 16),
                                           __uint_as_float(vh.y & 0xffff0000u)};
                             if (kConv || m > 0) {
-                                const uint2 vl = *reinterpret_cast<const uint2 *>(a_rl + off);
+                                const uint2 vl = ld_shared8(a_rl + off);
                                 fadd2(x[0], x[1], x[0], x[1], __uint_as_float(vl.x << 16), __uint_as_float(vl.x & 0xffff0000u));
                                 fadd2(x[2], x[3], x[2], x[3], __uint_as_float(vl.y << 16), __uint_as_float(vl.y & 0xffff0000u));
                             }
