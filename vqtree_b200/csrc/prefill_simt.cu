@@ -1,8 +1,6 @@
 // Fused VQ-attention prefill, fp32 arithmetic on the regular cores (any activation dtype).
 //
-// This is the full-precision form of the fused kernel: it serves fp32 inputs (whose tolerance a
-// 16-bit tensor-core product cannot meet) and is the on-device cross-check of the tensor-core
-// kernel.  One warp owns one query row and runs ONE online softmax over, in this order,
+// The on-device cross-check of the tensor-core kernel and of the tiled fp32 kernel (prefill_f32.cu), for any type.  One warp owns one query row and runs ONE online softmax over, in this order,
 //   the far pseudo-keys   (q2 . codebook[r], weight cnt[r], value vsum[r])   ops/triton_fused_vq_attn.py:38-68
 //   the boundary keys     (q2 . k3)            ops/triton_fused_local_attn_rerope.py:68-75
 //   the window keys       (q1 . k1, causal)    ops/triton_fused_local_attn_rerope.py:45-49,76-78

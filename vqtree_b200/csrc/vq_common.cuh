@@ -69,7 +69,7 @@ inline int launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<Args &&>(args)...) == cudaSuccess ? VQ_OK : VQ_ELAUNCH;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Args &&>(args)...) == cudaSuccess ? launch_status() : (cudaGetLastError(), VQ_ELAUNCH);
 }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // lets the next kernel of the stream start its prologue (if it was launched with launch_overlapped)
