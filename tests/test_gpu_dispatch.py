@@ -137,3 +137,45 @@ def test_store_window_copies_and_zeroes(api, dtype, n, cap, D, pad):
     for s, w in zip(src, win):
         assert torch.equal(w[:, :, :n], s) and not w[:, :, n:].any()
     assert act is None or torch.equal(act, vs.to(dtype))
+
+
+# decode tiles start at row 0 for the rows before n_bd and at row n_bd for the others: edges of tiles on either side, nothing on
+# one side, nothing but far rows.  Reference: the same weights in fp32; P and the output are rounded to bf16 (2^-9 each of values
+# of order one), hence the 2e-2 of the bf16 bars.
+@pytest.mark.parametrize("n,n_bd,far", [(1, 0, False), (1, 1, True), (128, 127, True), (129, 128, False), (257, 1, True), (300, 129, True), (256, 256, True), (0, 0, True)])
+@pytest.mark.parametrize("G", [1, 4])
+def test_decode_rows_on_either_side_of_the_boundary(api, n, n_bd, far, G):
+    g = _gen(n * 7 + n_bd)
+    B, H, D, MK = 2, 3, 128, 256
+    q1, q2 = (_rn(g, B, H * G, D).bfloat16() for _ in range(2))
+    k1, k3, v = (_rn(g, B, H, n + 5, D).bfloat16() for _ in range(3))
+    act = _rn(g, H, MK, D).bfloat16() if far else None
+    cnt = torch.randint(0, 3, (B, H, MK), generator=g, device="cuda").float() if far else None
+    vs = (_rn(g, B, H, MK, D) * cnt[..., None]).bfloat16() if far else None
+    got = api.vq_attention_decode(q1, q2, k1, k3, v, act, cnt, vs, n_valid=n, n_bd=n_bd).float()
+    api.check_status()
+    q1f, q2f = (t.float().view(B, H, G, D) for t in (q1, q2))
+    s = [torch.einsum("bhgd,bhnd->bhgn", q2f, k3[:, :, :n_bd].float()), torch.einsum("bhgd,bhnd->bhgn", q1f, k1[:, :, n_bd:n].float())]
+    w, val = [torch.ones(B, H, n, device="cuda")], [v[:, :, :n].float()]
+    if far:
+        s.append(torch.einsum("bhgd,hnd->bhgn", q2f, act.float()).masked_fill((cnt == 0)[:, :, None], float("-inf")))
+        w.append(cnt)
+        val.append(vs.float())
+    p = torch.exp(torch.cat(s, -1) * D ** -0.5 - torch.cat(s, -1).amax(-1, keepdim=True) * D ** -0.5)
+    want = torch.einsum("bhgn,bhnd->bhgd", p, torch.cat(val, 2)) / (p * torch.cat(w, 2)[:, :, None]).sum(-1, keepdim=True)
+    assert (got.view(B, H, G, D) - want).abs().max() < 2e-2 * max(1.0, float(want.abs().max()))
+
+
+# four heads of a position per thread: head counts with a remainder, both memory orders, explicit positions; same bits as one tensor
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("Hq,Hkv,L,D", [(1, 1, 1, 64), (5, 3, 77, 128), (8, 4, 130, 64)])
+@pytest.mark.parametrize("heads_inner", [False, True])
+def test_rope_qk_equals_rope(api, dtype, Hq, Hkv, L, D, heads_inner):
+    g = _gen(Hq + L)
+    q, k = ((_rn(g, 2, L, H, D).transpose(1, 2) if heads_inner else _rn(g, 2, H, L, D)).to(dtype) for H in (Hq, Hkv))
+    pos = torch.randint(0, 500, (2, L), generator=g, device="cuda")
+    for positions in (None, pos):
+        q1, q2, k1 = api.rope_qk(q, k, positions, const_pos=300, n_pos=600, like_input=heads_inner)
+        w1, w2 = api.rope(q, positions, const_pos=300, n_pos=600)
+        assert torch.equal(q1, w1) and torch.equal(q2, w2) and torch.equal(k1, api.rope(k, positions, n_pos=600)[0])
+    api.check_status()
