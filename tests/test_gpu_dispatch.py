@@ -179,3 +179,53 @@ def test_rope_qk_equals_rope(api, dtype, Hq, Hkv, L, D, heads_inner):
         w1, w2 = api.rope(q, positions, const_pos=300, n_pos=600)
         assert torch.equal(q1, w1) and torch.equal(q2, w2) and torch.equal(k1, api.rope(k, positions, n_pos=600)[0])
     api.check_status()
+
+
+# the two forms of the 16-bit prefill (128-key steps; 64-key steps for short tiles on grids that fill the chip) on either side of
+# each line between them, ragged lengths, empty codes, grouped heads.  Reference: the fp32 row kernel; P and the output are rounded to
+# 8 (11) bits, hence the bars.
+@pytest.mark.parametrize("dtype,bar", [(torch.bfloat16, 2e-2), (torch.float16, 2.5e-3)])
+@pytest.mark.parametrize("B,Hq,Hkv,L,W,MK,D", [(1, 1, 1, 100, 128, 128, 64), (2, 2, 1, 129, 128, 128, 128), (1, 4, 2, 700, 128, 256, 128), (1, 3, 3, 1025, 256, 640, 64),
+                                               (3, 32, 8, 300, 128, 128, 128), (2, 16, 4, 1200, 128, 1536, 128), (2, 16, 4, 1200, 128, 1536, 64), (2, 24, 4, 577, 256, 256, 64)])
+@pytest.mark.parametrize("rerope", [False, True])
+def test_prefill_forms_agree_with_the_row_kernel(api, dtype, bar, B, Hq, Hkv, L, W, MK, D, rerope):
+    g = _gen(L + MK)
+    q1, q2 = (_rn(g, B, Hq, L, D).to(dtype) for _ in range(2))
+    k1, k3, v = (_rn(g, B, Hkv, L, D).to(dtype) for _ in range(3))
+    if not rerope:
+        q2, k3 = q1, k1
+    nb = api.far_blocks(L, W)
+    act = cnt = vs = None
+    if nb:
+        act = (_rn(g, Hkv, MK, D) * D ** -0.25).to(dtype)
+        cnt = torch.randint(0, 4, (B, Hkv, nb, MK), generator=g, device="cuda").float()
+        vs = (_rn(g, B, Hkv, nb, MK, D) * cnt[..., None]).to(dtype)
+    got, lse = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True)
+    want, lse_w = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True, impl="simt")
+    api.check_status()
+    assert (got.float() - want.float()).abs().max() <= bar * max(1.0, float(want.float().abs().max())) and (lse - lse_w).abs().max() < 1e-4
+
+
+# a row whose largest score lies in the second half of its first 128 keys, up to 2^8 above the first half's: its weight is exactly one,
+# so that a value met by that key alone comes out as the correctly rounded 1 / (1 + (keys - 1) 2^-x).  Rounding that weight as well adds
+# up to half a unit in the last place.  128 CTAs: steps of 128 keys; 512: of 64.
+@pytest.mark.parametrize("B", [1, 4])
+@pytest.mark.parametrize("dtype,ulp", [(torch.bfloat16, 2.0 ** -7), (torch.float16, 2.0 ** -10)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("rerope", [False, True])
+def test_prefill_largest_weight_is_one(api, B, dtype, ulp, D, rerope):
+    H, L = 64, 256
+    q1 = torch.zeros(B, H, L, D, device="cuda", dtype=dtype)
+    q1[..., 0] = 1
+    k1 = torch.zeros(B, H, L, D, device="cuda", dtype=dtype)
+    k1[:, :, 100, 0] = torch.linspace(1.0, 7.9, B * H, device="cuda").view(B, H).to(dtype)
+    v = torch.zeros_like(k1)
+    v[:, :, 100] = 1
+    scale = 1 / 1.4426950408889634
+    q2, k3 = (q1.clone(), k1.clone()) if rerope else (q1, k1)
+    out = api.prefill_from_aggregates(q1, q2, k1, k3, v, None, None, None, 256, scale=scale)
+    api.check_status()
+    for row in (127, 255):
+        want = 1 / (1 + row * torch.exp2(-k1[:, :, 100, 0].double()))
+        err = (out[:, :, row].double() / want[..., None] - 1).abs().max()
+        assert err <= 0.5 * ulp * (1 + 2.0 ** -8) + 1e-6, float(err / ulp)   # half a unit at the bottom of a binade; sums and exponentials are fp32
