@@ -92,11 +92,10 @@ __device__ __forceinline__ float t4_max(const uint32_t (&r)[64])
 }
 
 // P = exp2(S * scale - m) of the 64 scores, packed 16-bit floats written to the 32 columns at p_addr; returns
-// the (FAR: count-weighted) sum of the 64 values.
+// sum plus the (FAR: count-weighted) sums of the two halves, one after the other.
 template <bool FAR, bool F16>
-__device__ __forceinline__ float t4_exp(const uint32_t (&r)[64], uint32_t p_addr, const float *cw, float scale_log2, float neg_m)
+__device__ __forceinline__ float t4_exp(const uint32_t (&r)[64], uint32_t p_addr, const float *cw, float scale_log2, float neg_m, float sum)
 {
-    float sum = 0.f;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         float ls[4] = {0.f, 0.f, 0.f, 0.f};
@@ -450,8 +449,8 @@ prefill_tc4_kernel(const __grid_constant__ CUtensorMap tm_q1, const __grid_const
 #pragma unroll
             for (int c = 0; c < KEYS; c += 64) {
                 if (KEYS > 64) t4_scores(sa + c, kind, has_empty, lo - c, hi - c, cw + c, r);
-                ls += kind == kFar ? t4_exp<true, F16>(r, sa + c / 2, cw + c, p.scale_log2, -m_safe)
-                                   : t4_exp<false, F16>(r, sa + c / 2, cw + c, p.scale_log2, -m_safe);
+                ls = kind == kFar ? t4_exp<true, F16>(r, sa + c / 2, cw + c, p.scale_log2, -m_safe, ls)
+                                  : t4_exp<false, F16>(r, sa + c / 2, cw + c, p.scale_log2, -m_safe, ls);
             }
             l_part += ls;
             tc_wait_st();
