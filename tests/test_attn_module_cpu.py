@@ -76,6 +76,17 @@ def test_use_rerope_restores_the_class():
     assert after is before
 
 
+def test_update_prefill_of_fake_tensors():
+    # shapes are propagated without a device: the kernel that stores real windows must not be handed storage that is not there
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    c = VectorQuantizedReRoPECache(128, torch.zeros(2, 1, 128, 64))
+    with FakeTensorMode():
+        k, raw, v = (torch.empty(1, 2, 100, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3))
+        cnt, vs = torch.empty(1, 2, 128, device="cuda"), torch.empty(1, 2, 128, 64, device="cuda")
+        c.update_prefill(cnt, vs, k, v, 0, 100, {"key_unrotated": raw})
+        assert c.key_buffers[0].shape == k.shape and c.states[0]["vsum"].dtype == torch.bfloat16 and c.seen_tokens == 100
+
+
 def test_codebook_pickle_roundtrip_and_errors(tmp_path):
     # the structure build_quantizer/120_build_additive_quantizer.py:60-66 writes: {(layer, head): [M arrays [K, D]]}
     rng = np.random.default_rng(0)

@@ -139,6 +139,32 @@ def test_store_window_copies_and_zeroes(api, dtype, n, cap, D, pad):
     assert act is None or torch.equal(act, vs.to(dtype))
 
 
+# what a prefill leaves in the cache when its tensors carry tangents, are negated lazily, or have no rows
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_update_prefill_of_tensors_that_a_kernel_cannot_read(dtype):
+    from torch.autograd import forward_ad as fw
+
+    from vqtree_b200.attn_vq import VectorQuantizedReRoPECache
+    g = _gen(3)
+    k, raw, v, tan = (_rn(g, 2, 2, 100, 64).to(dtype) for _ in range(4))
+    cnt, vs = _rn(g, 2, 2, 128), _rn(g, 2, 2, 128, 64)
+
+    def cache():
+        return VectorQuantizedReRoPECache(128, torch.zeros(2, 1, 128, 64, device="cuda"))
+
+    c = cache()
+    with fw.dual_level():
+        c.update_prefill(cnt, vs, fw.make_dual(k, tan), v, 0, 100, {"key_unrotated": raw})
+        got = fw.unpack_dual(c.key_buffers[0])
+        assert torch.equal(got.primal, k) and torch.equal(got.tangent, tan)
+    c = cache()
+    c.update_prefill(cnt, vs, torch._neg_view(k), v, 0, 100, {"key_unrotated": raw})
+    assert torch.equal(c.key_buffers[0], -k)
+    c = cache()
+    c.update_prefill(cnt[:0], vs[:0], k[:0], v[:0], 0, 100, {"key_unrotated": raw[:0]})
+    assert c.key_buffers[0].shape == (0, 2, 100, 64)
+
+
 # decode tiles start at row 0 for the rows before n_bd and at row n_bd for the others: edges of tiles on either side, nothing on
 # one side, nothing but far rows.  Reference: the same weights in fp32; P and the output are rounded to bf16 (2^-9 each of values
 # of order one), hence the 2e-2 of the bf16 bars.

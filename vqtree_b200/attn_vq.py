@@ -54,6 +54,22 @@ def rope_cos_sin(n_pos: int, dim: int, device, base: float = 10000.0):
     return ang.cos().float(), ang.sin().float()
 
 
+def _plain_cuda(*tensors) -> bool:
+    """True when a kernel may be handed the tensors' storage: CUDA memory that holds the values as they are (no fake, subclassed,
+    functorch-wrapped or lazily negated tensor), no derivative followed (either mode), nothing tracing the operators of this call."""
+    if torch._C._len_torch_dispatch_stack() or torch.jit.is_tracing() or torch.compiler.is_compiling():
+        return False
+    dual = torch.autograd.forward_ad
+    for t in tensors:
+        if not t.is_cuda or type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_functorch_wrapped_tensor(t) or t.is_neg():
+            return False
+        if t.requires_grad and torch.is_grad_enabled():
+            return False
+        if dual._current_level >= 0 and dual.unpack_dual(t).tangent is not None:
+            return False
+    return True
+
+
 class VectorQuantizedReRoPECache(_HFCache):
     """The object the reference passes as ``past_key_value`` (ops/attn_vq.py:31-52), with a working update.
 
@@ -178,15 +194,15 @@ class VectorQuantizedReRoPECache(_HFCache):
         srcs = (local_key, raw, local_value)
         vs32 = cumulated_value.float().contiguous()
         vsum = None
-        if (dt in (torch.float16, torch.bfloat16, torch.float32) and n_local > 0 and vs32.dim() == 4 and vs32.numel() % 4 == 0
-                and all(t.is_cuda and t.device == dev and t.dtype == dt and t.shape == local_key.shape and t.stride(-1) == 1
-                        and not (t.requires_grad and torch.is_grad_enabled()) for t in srcs)
-                and vs32.device == dev and vs32.data_ptr() % 16 == 0 and not (vs32.requires_grad and torch.is_grad_enabled())):
+        if (dt in (torch.float16, torch.bfloat16, torch.float32) and local_key.numel() > 0 and vs32.dim() == 4 and vs32.numel() > 0
+                and vs32.numel() % 4 == 0 and _plain_cuda(*srcs, vs32)
+                and all(t.device == dev and t.dtype == dt and t.shape == local_key.shape and t.stride(-1) == 1 for t in srcs)
+                and vs32.device == dev and vs32.data_ptr() % 16 == 0):
             bufs = [torch.empty(B, Hkv, cap, D, dtype=dt, device=dev) for _ in range(3)]
             if dt != torch.float32:
                 vsum = torch.empty(vs32.shape, dtype=dt, device=dev)
             api.store_window(*srcs, *bufs, vs32 if vsum is not None else None, vsum)
-        else:                                               # host tensors, mixed types, tracked gradients
+        else:                                               # host, fake and wrapped tensors, mixed types, tracked derivatives, no rows
             bufs = [torch.zeros(B, Hkv, cap, D, dtype=dt, device=dev) for _ in range(3)]
             for buf, src in zip(bufs, srcs):
                 buf[:, :, :n_local] = src
