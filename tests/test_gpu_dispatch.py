@@ -59,6 +59,33 @@ def test_assign_extreme_keys_equal_the_exact_kernel(api, dtype, M, K):
     assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
 
 
+# keys that tie with many codes: zero keys (padding; their code is 0 without a second look) among others, with the first codeword finite
+# or not and with a bias; collapsed codebooks, where more keys have a whole codebook to score than is done one by one
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("D,M,K", [(64, 3, 128), (128, 2, 256), (128, 1, 1024), (64, 2, 512)])
+def test_assign_tied_keys_equal_the_exact_kernel(api, dtype, D, M, K):
+    g = _gen(D + K)
+    L = 1381
+    cb = _rn(g, 2, M, K, D) * D ** -0.25
+    k = _rn(g, 2, L, 2, D).to(dtype).transpose(1, 2)
+    k[:, :, L // 3: L // 2] = 0
+    k[:, :, L // 2, D - 1] = -0.0
+    k[:, 1, 7] = 0
+    k[:, 1, 7, 5] = 6e-8 if dtype == torch.float16 else 1e-30      # not zero, though its square is
+    bad = cb.clone()
+    bad[:, 0, 0, 3] = float("nan")
+    bad[1, 0, 1, 3] = float("inf")
+    flat = cb.clone()
+    flat[:, :, :] = flat[:, :, :1]
+    flat[:, :, K // 2:, 0] += 2.0 ** -20
+    bias = _rn(g, 2, M, K)
+    for books, b in ((cb, None), (bad, None), (flat, None), (torch.zeros_like(cb), None), (cb, bias), (flat, bias * 0)):
+        got = api.assign_codes(k, books, b, out_dtype=torch.int32)
+        want = api.assign_codes(k, books, b, out_dtype=torch.int32, impl="simt")
+        api.check_status()
+        assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
+
+
 # sorted aggregates of half and fp32 values: the same sums bit for bit as the kernel without a workspace
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("L,D,M,K", [(128, 64, 1, 128), (390, 128, 2, 256), (1024, 64, 3, 64), (640, 128, 1, 1024)])

@@ -385,6 +385,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
         float4 *xch = &s_x[s][row];
         float rbound;  // |k| + sum of the largest codeword norms so far: a priori bound of the residual's norm
         float rnow;    // bound of the current residual's norm (tighter): see the residual update below
+        bool zero_key;  // every element is zero (padding): see `tied` below
         bool ok = true;
         if constexpr (kConv) {
             // ---- the keys of this stream as two bf16 terms in the operand layout, and their squared norms.  As in the
@@ -410,6 +411,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 }
                 store_terms(a_rh, a_rl, lane_off + r * 128 + ((chunk ^ (r & 7)) << 4), x);
                 float ss = fmaf(x[0], x[0], fmaf(x[1], x[1], fmaf(x[2], x[2], x[3] * x[3])));
+                if constexpr (std::is_same<KT, float>::value)   // where only the squares vanish: not zero
+                    ss += fminf(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))), 1e-44f);
 #pragma unroll
                 for (int off = LPR / 2; off >= 1; off >>= 1) ss += __shfl_xor_sync(kAll, ss, off);
                 if (l == 0) s_norm2[s][r] = ss;
@@ -418,15 +421,18 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             mbar_arrive(&bar_q[s]);
             ok = __all_sync(kAll, mbar_wait(&bar_q[s], 0, p.wait_limit));   // every warp's part, this row's norm among them
             rbound = sqrtf(fmaxf(s_norm2[s][row], kAtMinNorm2)) * 1.0001f;
+            zero_key = s_norm2[s][row] == 0.f;
             rnow = rbound;
         } else {
             ok = __all_sync(kAll, mbar_wait(&bar_k[s], 0, p.wait_limit));
             // |k| from the key tile the TMA load put into shared memory (this thread's row, 16-byte chunks in the
             // 128-byte swizzle: eight consecutive rows read eight different chunks, so the reads do not collide)
             float ss = 0.f;
+            uint32_t any = 0;
 #pragma unroll 4
             for (int ck = 0; ck < D / 8; ++ck) {
                 const uint4 raw = *reinterpret_cast<const uint4 *>(a_tile + (ck >> 3) * kHalfBytes + row * 128 + (((ck & 7) ^ (row & 7)) << 4));
+                any |= raw.x | raw.y | raw.z | raw.w;
                 const __nv_bfloat162 *hp = reinterpret_cast<const __nv_bfloat162 *>(&raw);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -436,6 +442,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             }
             rbound = sqrtf(fmaxf(ss, kAtMinNorm2)) * 1.0001f;
             rnow = rbound;
+            zero_key = (any & 0x7fff7fffu) == 0u;
         }
         uint32_t doubt = 0;   // bit m: the lead of codebook m's best score did not prove its arg-max (bit 8 + m: no record)
         uint32_t last_rec = 0xffffffffu;   // the key's most recent candidate record
@@ -447,6 +454,9 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             const float eps_m = (4.f + D / 64 + (splits > 0 ? 3 : 2) * (D / 32) + 1.1f * splits) * 3.814697265625e-6f;
             const float thr0 = 2.f * eps_m * rnow * cm + 1e-30f;
             const float *bm = p.bias ? p.bias + (static_cast<int64_t>(h) * M + m) * K : nullptr;
+            // A key of zeros scores +0 with every code whose entries are finite (NaN with the others): without a bias the
+            // first code is its arg-max if that code is finite, and no lead has to prove it.
+            const bool tied = m == 0 && zero_key && bm == nullptr && __ldg(p.cn2 + static_cast<int64_t>(h) * MK) < INFINITY;
             // ---- scan of this thread's groups, chunk by chunk as the tensor pipe finishes them: best and runner-up
             // of the tagged scores (the tag of the best gives its index inside its group of 32)
             float best = -INFINITY, second = -INFINITY;
@@ -482,7 +492,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 best = fmaxf(best, hi);
                 if constexpr (wrap) {
                     // a group whose runner-up came near gives up its third as well: there is no second look later
-                    const bool near_best = lo >= best - thr0;
+                    const bool near_best = valid && !tied && lo >= best - thr0;   // (rows past the end are zeros as well)
                     if (__any_sync(kAll, near_best)) {
                         load_scores(tbase + col, bm, 32 * g, v);
                         float g3 = -INFINITY;
@@ -568,12 +578,13 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                     third = fmaxf(third, oy.x);
                 }
                 code = bgrp * 32 + 31 - static_cast<int>(__float_as_uint(best) & 31u);  // first group holding the maximum
+                if (tied) code = 0;
                 *xch = make_float4(best, __int_as_float(code), 0.f, 0.f);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&x_done[s][wq]);
                 // with a bias the fp32 additions s + bias round by up to 2^-24 |s + bias| each
                 const float thr = bm ? thr0 + fabsf(best) * 4.76837158203125e-7f : thr0;
-                const bool dflag = valid && !(best - second > thr);
+                const bool dflag = valid && !tied && !(best - second > thr);
                 if (__ballot_sync(kAll, dflag)) {
                     // ---- some key of this warp is doubtful: its candidates (scores within thr of the best) go into a
                     // record for the repair kernel; carry on with the approximate winner.  The best and the runner-up are
@@ -911,9 +922,140 @@ __device__ __forceinline__ uint32_t settle_key(const AtParams &p, const uint4 en
     return 0u;
 }
 
+// Every key of the call, exactly, in tiles of 32 keys that share the codebook rows: for calls where so many keys tie (equal or
+// collapsed codewords, residuals of zero) that scoring a codebook once per such key costs more than once per tile.  Thread (kq, cr)
+// scores keys 4 kq .. 4 kq + 3 against codes cr, cr + 16, cr + 32, cr + 48 of 64 codewords, a quarter of whose columns is in shared
+// memory at a time.  Bound by shared-memory loads (eight of 16 bytes per 64 FMAs).
+constexpr int kBulkKeys = 32, kBulkCodes = 64;
 template <typename KT, int D>
-__global__ void __launch_bounds__(kAtRepairWarps * 32)
-assign_repair_kernel(AtParams p)
+__device__ __noinline__ void settle_all(const AtParams &p, float *mem)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int DC = D / 4, CP = DC + 4;   // columns at a time; floats per staged row (padded: a warp's four rows lie in different banks)
+    static_assert(kAtRepairWarps * 32 == kBulkKeys / 4 * 16, "thread (kq, cr)");
+    float *rT = mem, *cw = rT + D * kBulkKeys;                                         // residuals [D][keys], codewords [64][DC]
+    int *s_code = reinterpret_cast<int *>(cw + kBulkCodes * CP);
+    float *s_v = cw;                                                                   // best scores [warp][key] and their codes, over the codewords
+    int *s_i = reinterpret_cast<int *>(s_v + kAtRepairWarps * kBulkKeys);
+    static_assert(sizeof(float) * (D * kBulkKeys + kBulkCodes * CP + kBulkKeys) <= kAtRepairWarps * sizeof(AtRepairBuf<D>), "shared memory");
+    const int tid = threadIdx.x, warp = tid >> 5, kq = tid & 7, cr = tid >> 3;
+    const int M = p.M, K = p.K;
+    const int64_t per_unit = (p.L + kBulkKeys - 1) / kBulkKeys, tiles = p.pool_cap / p.L * per_unit;
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int u = static_cast<int>(t / per_unit), b = u / p.Hkv, h = u % p.Hkv;
+        const int64_t j0 = t % per_unit * kBulkKeys;
+        const KT *kb = static_cast<const KT *>(p.k) + b * p.k_sb + h * p.k_sh;
+        __syncthreads();           // the previous tile's reads
+        for (int e = tid; e < kBulkKeys * D; e += kAtRepairWarps * 32) {
+            const int key = e / D, d = e % D;
+            rT[d * kBulkKeys + key] = j0 + key < p.L ? to_f32(kb[(j0 + key) * p.k_sl + d]) : 0.f;
+        }
+        for (int m = 0; m < M; ++m) {
+            const float *cm = p.cb + (static_cast<int64_t>(h) * M + m) * K * D;
+            const float *bm = p.bias ? p.bias + (static_cast<int64_t>(h) * M + m) * K : nullptr;
+            float bv[4];
+            int bi[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                bv[i] = -INFINITY;
+                bi[i] = 0;         // no score above -inf (NaN scores): the first code, as in the exact kernel
+            }
+            for (int c0 = 0; c0 < K; c0 += kBulkCodes) {   // (K is a multiple of 128)
+                float acc[4][4];   // [code][key]
+#pragma unroll
+                for (int i = 0; i < 16; ++i) acc[i >> 2][i & 3] = 0.f;
+#pragma unroll 1
+                for (int d0 = 0; d0 < D; d0 += DC) {
+                    __syncthreads();   // residuals written, the previous rows read
+#pragma unroll
+                    for (int i = 0; i < kBulkCodes * DC / 4 / (kAtRepairWarps * 32); ++i) {
+                        const int e = tid + i * kAtRepairWarps * 32, c = e / (DC / 4), q = e % (DC / 4);
+                        *reinterpret_cast<float4 *>(cw + c * CP + 4 * q) = __ldg(reinterpret_cast<const float4 *>(cm + static_cast<int64_t>(c0 + c) * D + d0) + q);
+                    }
+                    __syncthreads();
+#pragma unroll 1
+                    for (int d = 0; d < DC; d += 4) {
+                        float cv[4][4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const float4 c4 = *reinterpret_cast<const float4 *>(cw + (cr + 16 * i) * CP + d);
+                            cv[i][0] = c4.x; cv[i][1] = c4.y; cv[i][2] = c4.z; cv[i][3] = c4.w;
+                        }
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float4 r4 = *reinterpret_cast<const float4 *>(rT + (d0 + d + e) * kBulkKeys + 4 * kq);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                acc[i][0] = __fmaf_rn(r4.x, cv[i][e], acc[i][0]);
+                                acc[i][1] = __fmaf_rn(r4.y, cv[i][e], acc[i][1]);
+                                acc[i][2] = __fmaf_rn(r4.z, cv[i][e], acc[i][2]);
+                                acc[i][3] = __fmaf_rn(r4.w, cv[i][e], acc[i][3]);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int c = c0 + cr + 16 * i;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float sc = bm ? __fadd_rn(acc[i][k], __ldg(bm + c)) : acc[i][k];
+                        if (sc > bv[k]) {      // a thread's codes come in increasing order: the first maximum stays
+                            bv[k] = sc;
+                            bi[k] = c;
+                        }
+                    }
+                }
+            }
+            __syncthreads();       // the last codewords have been read: the bests go over them
+            auto take = [](float &v, int &i, float ov, int oi) {
+                if (ov > v || (ov == v && oi < i)) {
+                    v = ov;
+                    i = oi;
+                }
+            };
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                for (int off = 16; off >= 8; off >>= 1) {
+                    const float ov = __shfl_xor_sync(kAll, bv[i], off);
+                    const int oi = __shfl_xor_sync(kAll, bi[i], off);
+                    take(bv[i], bi[i], ov, oi);
+                }
+                if ((tid & 31) < 8) {
+                    s_v[warp * kBulkKeys + 4 * kq + i] = bv[i];
+                    s_i[warp * kBulkKeys + 4 * kq + i] = bi[i];
+                }
+            }
+            __syncthreads();
+            if (tid < kBulkKeys) {
+                float v = s_v[tid];
+                int c = s_i[tid];
+#pragma unroll
+                for (int w = 1; w < kAtRepairWarps; ++w) take(v, c, s_v[w * kBulkKeys + tid], s_i[w * kBulkKeys + tid]);
+                s_code[tid] = c;
+                if (j0 + tid < p.L) store_code(p.codes, p.code_dtype, b * p.c_sb + h * p.c_sh + (j0 + tid) * p.c_sl + m, c);
+            }
+            if (m + 1 < M) {
+                __syncthreads();
+                const int key = tid & (kBulkKeys - 1);
+                const float *crow = cm + static_cast<int64_t>(s_code[key]) * D;
+                for (int q = warp; q < D / 4; q += kAtRepairWarps) {
+                    const float4 x = __ldg(reinterpret_cast<const float4 *>(crow) + q);
+                    float *r = rT + 4 * q * kBulkKeys + key;
+                    r[0] = __fsub_rn(r[0], x.x);
+                    r[kBulkKeys] = __fsub_rn(r[kBulkKeys], x.y);
+                    r[2 * kBulkKeys] = __fsub_rn(r[2 * kBulkKeys], x.z);
+                    r[3 * kBulkKeys] = __fsub_rn(r[3 * kBulkKeys], x.w);
+                }
+            }
+        }
+    }
+}
+
+template <typename KT, int D>
+__global__ void __launch_bounds__(kAtRepairWarps * 32, 6)
+assign_repair_kernel(const __grid_constant__ AtParams p)
 {
     __shared__ __align__(16) AtRepairBuf<D> s_buf[kAtRepairWarps];
     __shared__ float2 s_team[kAtRepairWarps];
@@ -921,6 +1063,14 @@ assign_repair_kernel(AtParams p)
     __shared__ unsigned int s_nleft;
     const int warp = threadIdx.x >> 5;
     const unsigned int count = p.counters[0], heavy = p.counters[2];
+    // Past this many keys with a whole codebook to score, all keys are scored in tiles (every CTA reads the same counter).  Such a
+    // key takes the chip 0.07 us (K = 256) to 0.22 us (K = 1024) by itself, any key 10 ns per 1024 codes in a tile; up to two per
+    // CTA they are short beside a tile's latency.  32 heads x 5001 keys, all codewords equal, M1 K1024: 40.5 -> 1.7 ms (the
+    // exact kernel: 1.4 ms).  `p` is passed on by reference: as a plain parameter its copy in local memory cost every call 2 - 3 us.
+    if (heavy > max(p.pool_cap / 24u, 2u * gridDim.x)) {
+        settle_all<KT, D>(p, reinterpret_cast<float *>(s_buf));
+        return;
+    }
     if (threadIdx.x == 0) s_nleft = 0u;
     __syncthreads();
     // the long ones first: they are spread over all CTAs
