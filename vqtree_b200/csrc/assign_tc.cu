@@ -1179,7 +1179,10 @@ extern "C" int vqattn_assign_codes_ws(const VqTensorDesc *k, const VqTensorDesc 
     // Few keys against few codewords: the exact kernel is one launch of a short chain, this path four (codebook split, scan,
     // repair, a memset).  Measured (us, this path / exact kernel): M*K*D = 8192: 8192 keys 25 / 11, 32768 keys 26 / 25;
     // 16384: 8192 keys 28 / 17, 32768 keys 28 / 50; 32768: 256 keys 25 / 34, 32768 keys 35 / 84.
-    const bool small = shapes_ok && M * K * D <= (1 << 14) && k->shape[0] * k->shape[1] * k->shape[2] <= (1 << 14);
+    // M*K*D = 16384, 12288 keys, exact kernel / this path: M1 K128 25.6 / 20.5 (half 25.6 / 23.5), M2 K128 27.2 / 24; so the line runs
+    // through the product as well.
+    const int64_t keys = shapes_ok ? k->shape[0] * k->shape[1] * k->shape[2] : 0;
+    const bool small = shapes_ok && M * K * D <= (1 << 14) && keys <= (1 << 14) && keys * (M * K * D) <= (int64_t(1) << 27);
     // half and fp32 keys without a (sufficient) workspace take the exact kernel as well
     const bool ws_ok = workspace != nullptr && reinterpret_cast<uintptr_t>(workspace) % 256 == 0 && shapes_ok &&
                        workspace_bytes >= vqattn_assign_workspace_bytes(k->shape[0], k->shape[1], k->shape[2], M, K, D);
