@@ -202,8 +202,11 @@ __global__ void gather_aggregates_kernel(const T *__restrict__ v_vq, int64_t s_b
 // Rows moved as 16-byte vectors: LPR lanes per row, kGatherRows rows in flight per lane group (index and count loads of
 // all of them first, then the row loads, then the streaming stores).  Bound by the snapshot writes (the source array is
 // read many times and stays in L2).  B1 H32 D128, 56 blocks x 1024 codes, bf16 (0.47 GB written): 127 us; one element per
-// lane and instruction, one row per warp at a time (the kernel above, kept for rows that are no multiple of 16 bytes): 431 us.
+// lane and instruction, one row per warp at a time (the kernel above, kept for rows that are no multiple of 16 bytes and for
+// few rows, where more warps count): 431 us.  In us, this kernel / the one above, bf16, D = 128: 8192 rows 2.68 / 3.35, 4096
+// rows 2.68 / 2.46, 128 rows 2.41 / 2.00 (fp32 3.14 / 3.39, 2.74 / 2.52, 2.52 / 2.02).
 constexpr int kGatherRows = 4;
+constexpr int64_t kGatherFew = 4096;
 
 template <int LPR>
 __global__ void __launch_bounds__(256)
@@ -387,7 +390,13 @@ static int vq::build_aggregates_impl(const VqTensorDesc *codes, const VqTensorDe
         c2.shape[2] = v2.shape[2] = state_blocks * kBlock;
         return vqattn_cache_advance(&c2, &v2, K, state_cnt, state_vsum, nullptr, status_word, stream);
     }
-    if (NB > 0 && workspace != nullptr && aggregates_sorted_eligible(v, vsum, K) &&
+    // Half and fp32 values: over few blocks the one launch of the kernel below is shorter than sort and sums.  Measured (us, below /
+    // sorted): one block 3.5 - 6.7 / 5.7 - 8.0; M <= 2, three blocks 7.3 - 9.4 / 8.8 - 11.1, four 9.3 - 12.0 / 10.5 - 13.6, five 11.2 -
+    // 14.4 / 10.9 - 14.5, six 13.1 - 16.7 / 11.6 - 16.3; M = 4, 8: two 7.1 - 10.7 / 7.2 - 10.2, three 10.0 - 15.1 / 8.4 - 11.9.
+    // Snapshots of 8 MB a block (16 heads of 1024 codes, 128 fp32 columns), two blocks 8.8 - 10.7 / 9.5 - 9.9, four 15.8 - 19.1 / 13.3 - 13.9.
+    const int64_t block_bytes = B * Hkv * MK * D * (v->dtype == VQ_F32 ? 4 : 2);
+    const bool few = v->dtype != VQ_BF16 && NB <= (block_bytes > (int64_t(6) << 20) ? 1 : M <= 2 ? 4 : 2);
+    if (NB > 0 && !few && workspace != nullptr && aggregates_sorted_eligible(v, vsum, K) &&
         workspace_bytes >= aggregates_sorted_workspace_bytes(B, Hkv, NB, M, K))
         return launch_aggregates_sorted(codes, v, K, cnt, vsum, workspace, status_word, static_cast<cudaStream_t>(stream));
     if (NB > 0 && aggregates_reg_eligible(v, vsum, K))
@@ -449,7 +458,7 @@ extern "C" int vqattn_gather_aggregates(const VqTensorDesc *v_vq, const VqTensor
     if (B * H > 65535) return VQ_EUNSUPPORTED;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t esize = v_vq->dtype == VQ_F32 ? 4 : 2, lpr = D * esize / 16;
-    const bool rows16 = D * esize % 16 == 0 && NB * C < (int64_t(1) << 31) && (lpr == 8 || lpr == 16 || lpr == 32) && reinterpret_cast<uintptr_t>(v_vq->ptr) % 16 == 0 &&
+    const bool rows16 = B * H * NB * C > kGatherFew && D * esize % 16 == 0 && NB * C < (int64_t(1) << 31) && (lpr == 8 || lpr == 16 || lpr == 32) && reinterpret_cast<uintptr_t>(v_vq->ptr) % 16 == 0 &&
                         reinterpret_cast<uintptr_t>(vsum->ptr) % 16 == 0 && v_vq->stride[0] * esize % 16 == 0 &&
                         v_vq->stride[1] * esize % 16 == 0 && v_vq->stride[2] * esize % 16 == 0;
     if (rows16) {
