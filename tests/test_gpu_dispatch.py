@@ -222,9 +222,9 @@ def test_decode_rows_on_either_side_of_the_boundary(api, n, n_bd, far, G):
     assert (got.view(B, H, G, D) - want).abs().max() < 2e-2 * max(1.0, float(want.abs().max()))
 
 
-# four heads of a position per thread: head counts with a remainder, both memory orders, explicit positions; same bits as one tensor
+# one head of a position per thread, or four (the last shape): head counts with a remainder, both memory orders, explicit positions; same bits as one tensor
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("Hq,Hkv,L,D", [(1, 1, 1, 64), (5, 3, 77, 128), (8, 4, 130, 64)])
+@pytest.mark.parametrize("Hq,Hkv,L,D", [(1, 1, 1, 64), (5, 3, 77, 128), (8, 4, 130, 64), (13, 6, 590, 128)])
 @pytest.mark.parametrize("heads_inner", [False, True])
 def test_rope_qk_equals_rope(api, dtype, Hq, Hkv, L, D, heads_inner):
     g = _gen(Hq + L)

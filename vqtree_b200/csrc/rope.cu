@@ -231,14 +231,15 @@ __global__ void __launch_bounds__(256) rope_multi_kernel(const RopeMultiParams p
     }
 }
 
-// The rotations of a prefill: the same work with kRopeHeads heads of one position per thread, whose table rows are loaded once
+// The rotations of a prefill: the same work with NHEADS heads of one position per thread, whose table rows are loaded once
 // and whose rows are in flight together, and with 32-bit index arithmetic (below 2^31 work items).  HBM-bound; the kernel
 // above, one row per thread behind five 64-bit divisions, was bound by its instructions (issue slots 53 %).
 // 2 x 131072 tokens, 32 + 8 heads of 128, two rotations of q (7.5 GB): 1842 -> 1421 us; 32 + 32 heads, 5001 tokens: 52 -> 39 us.
+// Four heads, or one where four would leave too few threads (see rope_heads_launch).
 constexpr int kRopeHeads = 4;
 
-template <typename T>
-__global__ void __launch_bounds__(256) rope_heads_kernel(const RopeMultiParams p)   // job.first, total: in units of kRopeHeads heads
+template <typename T, int NHEADS>
+__global__ void __launch_bounds__(256) rope_heads_kernel(const RopeMultiParams p)   // job.first, total: in units of NHEADS heads
 {
     constexpr int N = RopeVec<T>::kN;
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(256) rope_heads_kernel(const RopeMultiParams p
         if (t < p.njobs && i >= static_cast<uint32_t>(p.job[t].first)) j = t;
     const RopeJob &jb = p.job[j];
     const int half = p.D / 2;
-    const uint32_t tpr = half / N, groups = (jb.H + kRopeHeads - 1) / kRopeHeads, L = static_cast<uint32_t>(p.L);
+    const uint32_t tpr = half / N, groups = (jb.H + NHEADS - 1) / NHEADS, L = static_cast<uint32_t>(p.L);
     const uint32_t w = i - static_cast<uint32_t>(jb.first), r = w / tpr;
     const int d = static_cast<int>(w % tpr) * N;
     // rows in the order they lie in memory (see rope_kernel)
@@ -263,11 +264,11 @@ __global__ void __launch_bounds__(256) rope_heads_kernel(const RopeMultiParams p
         hg = (r / L) % groups;
         b = (r / L) / groups;
     }
-    const int h0 = static_cast<int>(hg) * kRopeHeads, nh = min(kRopeHeads, jb.H - h0);
+    const int h0 = static_cast<int>(hg) * NHEADS, nh = min(NHEADS, jb.H - h0);
     const T *xp = static_cast<const T *>(jb.x) + b * jb.x_sb + h0 * jb.x_sh + l * jb.x_sl + d;
-    uint4 raw[kRopeHeads][2];
+    uint4 raw[NHEADS][2];
 #pragma unroll
-    for (int k = 0; k < kRopeHeads; ++k)
+    for (int k = 0; k < NHEADS; ++k)
         if (k < nh) {
             raw[k][0] = *reinterpret_cast<const uint4 *>(xp + k * jb.x_sh);
             raw[k][1] = *reinterpret_cast<const uint4 *>(xp + k * jb.x_sh + half);
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(256) rope_heads_kernel(const RopeMultiParams p
         rope_table<N>(p.cos_tab + row * half + d, cv);
         rope_table<N>(p.sin_tab + row * half + d, sv);
 #pragma unroll
-        for (int k = 0; k < kRopeHeads; ++k)
+        for (int k = 0; k < NHEADS; ++k)
             if (k < nh) {
                 float x1[N], x2[N], o1[N], o2[N];
                 RopeVec<T>::load(reinterpret_cast<const T *>(&raw[k][0]), x1);
@@ -356,17 +357,27 @@ static int rope_multi_launch(const RopeMultiParams &p, int dtype, cudaStream_t s
 // rope_heads_kernel over the jobs of p where its 32-bit indices reach, else the kernel above
 static int rope_heads_launch(const RopeMultiParams &p, int64_t B, int dtype, int vec, cudaStream_t s)
 {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return VQ_EDEVICE;
+    // One head per thread while that makes no more than two CTAs per SM: 8 + 8 heads, 128 tokens, both rotations of q 2.63 us (four
+    // heads: 3.44; one row per thread, 64-bit: 3.01), 32 + 32 heads of 128 tokens 2.84 (3.57; 3.36), of 192: 3.35 (3.58; 3.95), 256: 3.81 (3.75; 4.40).
+    const int nheads = p.total <= int64_t(512) * sms ? 1 : kRopeHeads;
     RopeMultiParams g = p;
     g.total = 0;
     for (int j = 0; j < g.njobs; ++j) {
         g.job[j].first = g.total;
-        g.total += B * ((g.job[j].H + kRopeHeads - 1) / kRopeHeads) * g.L * (g.D / 2 / vec);
+        g.total += B * ((g.job[j].H + nheads - 1) / nheads) * g.L * (g.D / 2 / vec);
     }
     if (g.total == 0 || g.total >= (int64_t(1) << 31) - 256) return rope_multi_launch(p, dtype, s);
     const unsigned grid = static_cast<unsigned>((g.total + 255) / 256);
-    if (dtype == VQ_F32) rope_heads_kernel<float><<<grid, 256, 0, s>>>(g);
-    else if (dtype == VQ_F16) rope_heads_kernel<__half><<<grid, 256, 0, s>>>(g);
-    else rope_heads_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(g);
+    auto go = [&](auto elem) {
+        using T = decltype(elem);
+        if (nheads == 1) rope_heads_kernel<T, 1><<<grid, 256, 0, s>>>(g);
+        else rope_heads_kernel<T, kRopeHeads><<<grid, 256, 0, s>>>(g);
+    };
+    if (dtype == VQ_F32) go(float{});
+    else if (dtype == VQ_F16) go(__half{});
+    else go(__nv_bfloat16{});
     return launch_status();
 }
 
