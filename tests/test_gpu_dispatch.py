@@ -19,9 +19,10 @@ def _rn(g, *s):
     return torch.randn(*s, generator=g, device="cuda")
 
 
-# half and fp32 keys on the tensor cores (two bf16 terms from the start): the same codes as the exact kernel, whole numbers
+# half and fp32 keys on the tensor cores (two bf16 terms from the start): the same codes as the exact kernel, whole numbers; (127, 64, 2,
+# 128) is small enough to be handed to that kernel
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
-@pytest.mark.parametrize("L,D,M,K", [(1, 128, 1, 128), (127, 64, 2, 128), (385, 128, 2, 128), (129, 128, 4, 256), (257, 128, 8, 256), (700, 64, 3, 384),
+@pytest.mark.parametrize("L,D,M,K", [(1, 64, 3, 128), (127, 64, 2, 128), (127, 64, 3, 128), (515, 64, 3, 128), (1, 128, 2, 128), (640, 64, 2, 512), (513, 64, 2, 1024), (385, 128, 2, 128), (129, 128, 4, 256), (257, 128, 8, 256), (700, 64, 3, 384),
                                      (640, 128, 2, 512), (1025, 128, 1, 1024)])
 def test_assign_half_and_fp32_keys_equal_the_exact_kernel(api, dtype, L, D, M, K):
     g = _gen(L + K)
@@ -84,6 +85,21 @@ def test_assign_tied_keys_equal_the_exact_kernel(api, dtype, D, M, K):
         want = api.assign_codes(k, books, b, out_dtype=torch.int32, impl="simt")
         api.check_status()
         assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
+
+
+# more keys whose code the repair changes than a CTA can leave to its four warps (64 each): twins 2^-20 apart, of which the scan, whose
+# scores they share, takes the lower and the defining arithmetic the larger
+def test_assign_changes_more_codes_than_are_left_to_a_cta(api):
+    g = _gen(11)
+    cb = _rn(g, 8, 3, 128, 64) * 64 ** -0.25
+    cb[:, :, 1::2] = cb[:, :, 0::2] * (1 + 2.0 ** -20)
+    k = _rn(g, 1, 8, 24000, 64).bfloat16()
+    got = api.assign_codes(k, cb, out_dtype=torch.int32)
+    want = api.assign_codes(k, cb, out_dtype=torch.int32, impl="simt")
+    api.check_status()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert int((want[..., 0] % 2).sum()) > 64 * 8 * sms
+    assert torch.equal(got, want), f"{int((got != want).sum())} codes differ"
 
 
 # sorted aggregates of half and fp32 values: the same sums bit for bit as the kernel without a workspace
@@ -167,6 +183,17 @@ def test_store_window_copies_and_zeroes(api, dtype, n, cap, D, pad):
     for s, w in zip(src, win):
         assert torch.equal(w[:, :, :n], s) and not w[:, :, n:].any()
     assert act is None or torch.equal(act, vs.to(dtype))
+
+
+# indices past 32 bits: 3 x 2^31 / 3 single elements and more (5 GB in all)
+def test_store_window_past_32_bit_indices(api):
+    D, n = 41, 1 << 20
+    cap = (1 << 31) // (3 * D) + 1000
+    src = _rn(_gen(1), 1, 1, n, D).half()
+    win = [torch.full((1, 1, cap, D), 7.0, dtype=torch.half, device="cuda") for _ in range(3)]
+    api.store_window(src, src, src, *win)
+    for w in win:
+        assert torch.equal(w[:, :, :n], src) and int(w[:, :, n:].count_nonzero()) == 0
 
 
 # what a prefill leaves in the cache when its tensors carry tangents, are negated lazily, or have no rows

@@ -381,7 +381,8 @@ def test_errors_are_reported_not_crashed(api):
     (1, 4, 2048, 128, 4, 256),     # config 2 shape, scaled down
     (2, 2, 700, 128, 4, 512),      # config 4 codebooks (9-bit codes), ragged length
     (1, 2, 1024, 128, 8, 256),     # config 5 codebooks
-    (1, 3, 515, 64, 2, 128),       # D = 64
+    (1, 3, 515, 64, 2, 128),       # D = 64, small enough for the exact kernel
+    (1, 3, 515, 64, 3, 128),       # D = 64
     (1, 1, 128, 128, 1, 64),       # single chunk
     (1, 2, 900, 128, 3, 384),      # three 128-codeword chunks, one key tile per CTA
     (2, 1, 640, 64, 2, 512),       # D = 64 with 9-bit codes
