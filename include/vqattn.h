@@ -110,7 +110,8 @@ int vqattn_assign_codes(const VqTensorDesc *k, const VqTensorDesc *codebooks, co
  * codebook (and of half and fp32 keys), then an exact fp32 re-score of every key whose two best approximate
  * scores are closer than the proven error bound.  Needs `workspace` (256-byte aligned) of
  * vqattn_assign_workspace_bytes(B, Hkv, L, M, K, D) bytes for the split codebook.  Inputs outside the
- * tensor-core path (larger K or M; fp32 or f16 keys without a workspace) are forwarded to vqattn_assign_codes.
+ * tensor-core path (larger K or M; fp32 or f16 keys without a workspace) and small calls (few keys against few codewords,
+ * where one exact kernel is the shorter) are forwarded to vqattn_assign_codes.
  * `status_word`: device int32 or NULL, raised if a bounded device-side wait expires.
  */
 size_t vqattn_assign_workspace_bytes(int64_t B, int64_t Hkv, int64_t L, int64_t M, int64_t K, int64_t D);
@@ -135,7 +136,7 @@ int vqattn_build_aggregates(const VqTensorDesc *codes, const VqTensorDesc *v, in
  * 16-byte aligned; contents need not be preserved between calls): the keys of every 128-key block are sorted by
  * code once, so that the kernel that forms the sums reads each row's keys instead of scanning the block's codes.
  * Same results, bit for bit.  Used for values and sums of one type with D = 64 or 128 and K a multiple of 8 up to 4096
- * (half, fp32: K up to 256 or a multiple of it);
+ * (half, fp32: K up to 256 or a multiple of it, and more than a few blocks);
  * other inputs, a NULL workspace or one that is too small take the path of vqattn_build_aggregates.
  * A code outside [0, K) is left out and reported through status_word (VQ_WORD_BAD_CODE; may be NULL).
  */

@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from vqtree_b200.native import VqError
+
 pytestmark = pytest.mark.gpu
 
 
@@ -117,6 +119,12 @@ def test_sorted_aggregates_of_half_and_fp32_values(api, dtype, L, D, M, K):
     api.check_status()
     for a, p, b in zip(got[:2], plain, want):
         assert torch.equal(a, b) and torch.equal(p, b)
+    wrong = codes.clone()
+    wrong[1, 1, 100, 0] = K                                     # left out, and reported on either path
+    bad = api.build_aggregates(wrong, v, K, nb)
+    with pytest.raises(VqError):
+        api.check_status()
+    assert float(bad[0][:, :, -1].sum()) == float(plain[0][:, :, -1].sum()) - 1
     cnt, vs = torch.zeros_like(got[2]), torch.zeros_like(got[3])
     api.cache_advance(codes[:, :, : nb * 128], v[:, :, : nb * 128], K, cnt, vs)
     assert torch.equal(got[2], cnt) and torch.equal(got[3], vs)

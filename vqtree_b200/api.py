@@ -83,7 +83,7 @@ def assign_codes(k: torch.Tensor, codebooks: torch.Tensor, bias: Optional[torch.
                  workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Key -> code assignment (replaces ops/mini_vq.py:4-18; greedy residual for M > 1).
 
-    k [B,Hkv,L,D] f32|bf16, codebooks [Hkv,M,K,D] f32, bias None|[Hkv,M,K] f32 -> codes [B,Hkv,L,M].
+    k [B,Hkv,L,D] f32|f16|bf16, codebooks [Hkv,M,K,D] f32, bias None|[Hkv,M,K] f32 -> codes [B,Hkv,L,M].
     """
     dev = _require_cuda(k, codebooks, bias)
     B, Hkv, L, _ = k.shape
@@ -94,7 +94,7 @@ def assign_codes(k: torch.Tensor, codebooks: torch.Tensor, bias: Optional[torch.
         if impl == "simt":
             check(lib.vqattn_assign_codes(dk, dc, db if bias is not None else None, do, stream_ptr(dev)), "vqattn_assign_codes")
         else:
-            # tensor-core scoring + exact re-score where it applies (bf16 keys); same codes either way
+            # tensor-core scoring + exact re-score where it applies and pays; same codes either way
             need = lib.vqattn_assign_workspace_bytes(B, Hkv, L, M, K, k.shape[3])
             if workspace is None or workspace.numel() < need:
                 workspace = torch.empty(need, dtype=torch.uint8, device=dev)
@@ -284,7 +284,7 @@ def vq_attention_prefill(q1, q2, k1, k3, v, codebooks, window: int, scale: Optio
                          state_blocks: Optional[int] = None):
     """The whole prefill path: assign codes to k3, build aggregates of v, fused attention.
 
-    q1,q2 [B,Hq,L,D]; k1,k3,v [B,Hkv,L,D] (f32 or bf16); codebooks [Hkv,M,K,D] f32.
+    q1,q2 [B,Hq,L,D]; k1,k3,v [B,Hkv,L,D] (f32, f16 or bf16); codebooks [Hkv,M,K,D] f32.
     ReRoPE mode: q1,k1 rotated by position, q2 rotated to the constant position window+1, k3 un-rotated
     (ops/attn_vq.py:402-407).  Plain-RoPE mode: pass q2 = q1 and k3 = k1.
     All five may be strided views with a contiguous last dim, and so may ``out`` ([B,Hq,L,D] view of

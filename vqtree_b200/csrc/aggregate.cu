@@ -94,7 +94,8 @@ build_aggregates_kernel(const void *__restrict__ codes, int code_dtype, int64_t 
                         const TV *__restrict__ v, int64_t v_sb, int64_t v_sh, int64_t v_sl,
                         float *__restrict__ cnt,  // [B,Hkv,NB,MK] dense
                         TO *__restrict__ vsum,    // [B,Hkv,NB,MK,D] dense
-                        int Hkv, int D, int M, int K, int NB, int parts, int rows_per_part)
+                        int Hkv, int D, int M, int K, int NB, int parts, int rows_per_part,
+                        int32_t *__restrict__ status)   // nullptr, or raised for a code outside [0, K)
 {
     extern __shared__ __align__(16) float smem[];
     float *acc = smem;                               // [rows_per_part][32]
@@ -142,6 +143,7 @@ build_aggregates_kernel(const void *__restrict__ codes, int code_dtype, int64_t 
             const bool mine = local >= 0 && local < rows_per_part;
             s_code[tid] = mine ? local : -1;
             if (mine) atomicAdd(&s_cnt[local], 1);
+            if (status != nullptr && kp == 0 && ds == 0 && (ncode < 0 || ncode >= K)) atomicExch(status, VQ_WORD_BAD_CODE);
         }
 #pragma unroll
         for (int t = 0; t < kVecPerThread; ++t) {
@@ -417,7 +419,8 @@ static int vq::build_aggregates_impl(const VqTensorDesc *codes, const VqTensorDe
                                              codes->stride[2], static_cast<const TV *>(v->ptr), v->stride[0],         \
                                              v->stride[1], v->stride[2], static_cast<float *>(cnt->ptr),              \
                                              static_cast<TO *>(vsum->ptr), static_cast<int>(Hkv), static_cast<int>(D), \
-                                             static_cast<int>(M), static_cast<int>(K), static_cast<int>(NB), parts, rows); \
+                                             static_cast<int>(M), static_cast<int>(K), static_cast<int>(NB), parts, rows,   \
+                                             few ? status_word : nullptr);                                            \
     } while (0)
     if (v->dtype == VQ_F32 && vsum->dtype == VQ_F32) VQ_LAUNCH_AGG(float, float);
     else if (v->dtype == VQ_F16 && vsum->dtype == VQ_F16) VQ_LAUNCH_AGG(__half, __half);

@@ -25,27 +25,31 @@
 //   3. The other keys (well under one per cent of the (key, codebook) pairs for random data) keep the
 //      approximate winner for the time being.  Their candidates - the codes whose approximate score is
 //      within thr of the best; the exact arg-max is among them - are written to a record (up to four codes;
-//      more, as for an all-zero key, means "all of them"), the records of a key are chained, and the key
-//      goes on a work list.  A second, small kernel (assign_repair_kernel) walks the list: it follows the
+//      more means "all of them"), the records of a key are chained, and the key
+//      goes on a work list.  (A key of zeros ties with every finite code; its code is known without that.)  A second, small kernel (assign_repair_kernel) walks the list: it follows the
 //      key through the codebooks with the defining fp32 arithmetic, runs the defining chain for the
 //      candidates of every doubtful codebook (first maximum wins), and - in the rare case that this changes
 //      a code - recomputes every later codebook of that key over all its codewords, since its residual
-//      changed.  The scan kernel never waits for any of this.
+//      changed.  The scan kernel never waits for any of this.  Where too many keys have a whole codebook to score, the
+//      second kernel scores all keys instead, in tiles that share the codebook (settle_all).
 //      When a codebook is larger than the 256 score columns a stream owns in tensor memory (K = 512, 1024), its
 //      chunks pass through that region in rounds and the scores of a chunk are gone once the next one lands.  The
 //      candidates are then tracked during the scan: best, runner-up (each with its group of 32 codes) and the third
-//      largest of all group maxima and group runners-up.  If the third lies below the cut and no group's runner-up
-//      ever came within thr of the running best (the 30 unranked scores of a group are at most its runner-up, and
-//      the cut only rises with the running best), the best and the runner-up are the only candidates; otherwise,
-//      and always with a bias (thr then moves with the best score), the record says "all of them".
+//      largest of all group maxima and group runners-up - and, for a group whose runner-up came within thr of the
+//      running best, of the group's third score, looked up at once while it is there.  The cut only rises with the
+//      running best, so a third below it excludes every other code: a group that was not looked up has its runner-up,
+//      and with it its other 30 scores, below the cut.  Then the best and the runner-up are the only candidates;
+//      otherwise, and always with a bias (thr then moves with the best score), the record says "all of them".
+//      (Up to K = 384 the scores are still there: a group whose runner-up came near sets a flag, and such a key takes a
+//      second look.)
 // One CTA owns NS key tiles of 128 keys ("streams", NS = 2 except for K = 384): per stream eight warps,
 // two threads per key, each ranking half of the key's scores in tensor memory and updating half of
 // its residual row (the arithmetic between the MMAs is a chain of dependent instructions and loads
 // from L2: it needs the warps to hide its latency); one warp issues the MMAs of the streams in turn,
 // so the scan of one stream overlaps the MMAs of the other; one warp issues the TMA loads of the
 // codebook terms (16 KB units, 5-slot ring).  Every wait is bounded.
-// Half keys (B1 H32 D128 L5001, one codebook of 1024): 166 us + repair; on the exact kernel, which half and fp32 keys took
-// before, 1444 us.
+// Half keys (B1 H32 D128 L5001, one codebook of 1024), all kernels: 164 us; on the exact kernel, which half and fp32 keys took
+// before, 1440 us.
 #include <type_traits>
 
 #include "prefill_tc_common.cuh"
@@ -468,7 +472,7 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
             // threshold of the running best (the other 30 scores of such a group are unknown here and may hold further
             // candidates).  A doubtful key whose third lies below the cut needs no second look at its scores - which WRAP
             // could not take anyway: the scores of earlier chunks are gone by then, so there the third of such a group is
-            // looked up at once (M4 K512, 2 x 16384 tokens x 32 heads: 279 -> 115 us of repair, the scan stays at 1.49 ms).
+            // looked up at once (M4 K512, 2 x 16384 tokens x 32 heads: 279 -> 115 us of repair beside 1.38 ms of scan).
             float third = -INFINITY;
             int sgrp = g_lo;
             bool amb = bm != nullptr;   // with a bias the threshold moves with the best score: no short list then
@@ -588,8 +592,8 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant
                 if (__ballot_sync(kAll, dflag)) {
                     // ---- some key of this warp is doubtful: its candidates (scores within thr of the best) go into a
                     // record for the repair kernel; carry on with the approximate winner.  The best and the runner-up are
-                    // the only candidates when the third largest tracked score is below the cut and no group's runner-up
-                    // came near the best.  The other doubtful keys take a second look at their scores (tensor-memory
+                    // the only candidates when the third largest tracked score is below the cut (and, where the third of a close
+                    // group was not looked up, no group's runner-up came near the best).  The other doubtful keys take a second look at their scores (tensor-memory
                     // loads are warp-wide, so the warp re-reads the union of those keys' marked groups) - or, with WRAP,
                     // name every code a candidate (the repair kernel then scores the whole codebook).
                     const float cut = best - thr;
