@@ -643,8 +643,8 @@ def main():
         stages_ms=dict(assign_codes=stage_ms[0], build_aggregates=stage_ms[1], fused_attention=stage_ms[2]),
         roofline=dict(kernel="prefill_tc4_kernel (fused attention)", bound="tensor", achieved=attn_tflops, peak=peaks["tensor"],
                       unit="TFLOP/s", frac=attn_tflops / peaks["tensor"], peak_source=f"{peaks['source']} (burst bf16 matmul)",
-                      traffic=attention_bytes(w) * 1.012, traffic_unit="bytes per launch",
-                      traffic_note="algorithmic bytes x 1.012, the DRAM read+write / algorithmic ratio ncu measured on the c2 "
+                      traffic=attention_bytes(w) * 0.994, traffic_unit="bytes per launch",
+                      traffic_note="algorithmic bytes x 0.994, the DRAM read+write / algorithmic ratio ncu measured on the c2 "
                                    "capture; traffic grows in proportion to the (query tile, work item) pairs processed",
                       flops_per_launch=flops),
         stage_rooflines=stage_rooflines(w, stage_ms, peaks),

@@ -273,16 +273,20 @@ def test_rope_qk_equals_rope(api, dtype, Hq, Hkv, L, D, heads_inner):
 
 
 # the two forms of the 16-bit prefill (128-key steps; 64-key steps for short tiles on grids that fill the chip) on either side of
-# each line between them, ragged lengths, empty codes, grouped heads.  Reference: the fp32 row kernel; P and the output are rounded to
-# 8 (11) bits, hence the bars.
+# each line between them, ragged lengths, empty codes, grouped heads; keys that grow along the sequence, so that references are raised in
+# many items and in either half of one.  Reference: the fp32 row kernel; P and the output are rounded to 8 (11) bits, hence the bars.
+@pytest.mark.parametrize("growing", [False, True])
 @pytest.mark.parametrize("dtype,bar", [(torch.bfloat16, 2e-2), (torch.float16, 2.5e-3)])
 @pytest.mark.parametrize("B,Hq,Hkv,L,W,MK,D", [(1, 1, 1, 100, 128, 128, 64), (2, 2, 1, 129, 128, 128, 128), (1, 4, 2, 700, 128, 256, 128), (1, 3, 3, 1025, 256, 640, 64),
                                                (3, 32, 8, 300, 128, 128, 128), (2, 16, 4, 1200, 128, 1536, 128), (2, 16, 4, 1200, 128, 1536, 64), (2, 24, 4, 577, 256, 256, 64)])
 @pytest.mark.parametrize("rerope", [False, True])
-def test_prefill_forms_agree_with_the_row_kernel(api, dtype, bar, B, Hq, Hkv, L, W, MK, D, rerope):
+def test_prefill_forms_agree_with_the_row_kernel(api, dtype, bar, B, Hq, Hkv, L, W, MK, D, rerope, growing):
     g = _gen(L + MK)
     q1, q2 = (_rn(g, B, Hq, L, D).to(dtype) for _ in range(2))
     k1, k3, v = (_rn(g, B, Hkv, L, D).to(dtype) for _ in range(3))
+    if growing:
+        ramp = torch.linspace(0.05, 4.0, L, device="cuda")[:, None]
+        k1, k3 = (k1 * ramp).to(dtype), (k3 * ramp).to(dtype)
     if not rerope:
         q2, k3 = q1, k1
     nb = api.far_blocks(L, W)
@@ -294,7 +298,7 @@ def test_prefill_forms_agree_with_the_row_kernel(api, dtype, bar, B, Hq, Hkv, L,
     got, lse = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True)
     want, lse_w = api.prefill_from_aggregates(q1, q2, k1, k3, v, act, cnt, vs, W, return_lse=True, impl="simt")
     api.check_status()
-    assert (got.float() - want.float()).abs().max() <= bar * max(1.0, float(want.float().abs().max())) and (lse - lse_w).abs().max() < 1e-4
+    assert (got.float() - want.float()).abs().max() <= bar * max(1.0, float(want.float().abs().max())) and (lse - lse_w).abs().max() < 1e-4 * max(1.0, float(lse_w.abs().max()) / 10)
 
 
 # a row whose largest score lies in the second half of its first 128 keys, up to 2^8 above the first half's: its weight is exactly one,
