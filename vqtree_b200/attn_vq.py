@@ -54,18 +54,21 @@ def rope_cos_sin(n_pos: int, dim: int, device, base: float = 10000.0):
     return ang.cos().float(), ang.sin().float()
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
 def _plain_cuda(*tensors) -> bool:
-    """True when a kernel may be handed the tensors' storage: CUDA memory that holds the values as they are (no fake, subclassed,
-    functorch-wrapped or lazily negated tensor), no derivative followed (either mode), nothing tracing the operators of this call."""
-    if torch._C._len_torch_dispatch_stack() or torch.jit.is_tracing() or torch.compiler.is_compiling():
+    """True when a kernel may be handed the tensors' storage: CUDA memory that holds the values as they are (no fake, subclassed
+    or lazily negated tensor, no functorch transform under way), no derivative followed (either mode), nothing tracing the
+    operators of this call."""
+    if (torch._C._len_torch_dispatch_stack() or torch._C._functorch.peek_interpreter_stack() is not None or torch.jit.is_tracing()
+            or torch.compiler.is_compiling()):
         return False
-    dual = torch.autograd.forward_ad
+    grad, dual = torch.is_grad_enabled(), torch.autograd.forward_ad._current_level >= 0
     for t in tensors:
-        if not t.is_cuda or type(t) not in (torch.Tensor, torch.nn.Parameter) or torch._C._functorch.is_functorch_wrapped_tensor(t) or t.is_neg():
+        if type(t) not in _PLAIN or not t.is_cuda or t.is_neg() or (grad and t.requires_grad):
             return False
-        if t.requires_grad and torch.is_grad_enabled():
-            return False
-        if dual._current_level >= 0 and dual.unpack_dual(t).tangent is not None:
+        if dual and torch.autograd.forward_ad.unpack_dual(t).tangent is not None:
             return False
     return True
 
