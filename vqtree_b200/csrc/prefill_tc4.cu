@@ -25,10 +25,10 @@
 //               the query tile holds the constant-position queries first (far tiles, boundary block) and is reloaded with
 //               the rotated ones once the last score product that reads it has finished (64: shared memory for one).
 // What bounds it: no single unit, but the hand-offs of a step and, on short tiles, start and end of a CTA.  The 128-key form
-// reads a row's scores as two batches of 64 (one wait for each; batches of 32 were 1.12 times as long) in 128 registers without
-// spills; the 64-key form is held to 96 registers by its two CTAs and spills 64 - 76 bytes a thread.
-// B1 H32 L32768 W1024 MK1024, plain RoPE: 1.17 ms (batches of 32: 1.32, 64-key form 1.24); ReRoPE, B2 L16384 W512 MK2048: 1.68
-// ms (1.82, 1.78); half, L5001, MK1024: 206 us (229, 209).
+// reads a row's scores as two batches of 64 (one wait for each; four batches of 32: 1.24 -> 1.30 ms, B1 H32 L32768 W1024 MK1024, plain
+// RoPE, in turn on one card) in 128 registers without spills; the 64-key form is held to 96 registers by its two CTAs and spills
+// 64 - 76 bytes a thread.  128 / 64 keys in turn on one card: that shape 1.17 / 1.24 ms; ReRoPE, B2 L16384 W512 MK2048 1.68 /
+// 1.78 ms; half, ReRoPE, L5001, MK1024 206 / 209 us.
 // Hand-offs are mbarriers (tcgen05.commit arrives for the MMA side); every wait is bounded and a
 // failed wait raises the status word; all roles meet at one final barrier and TMEM is freed.
 #include "prefill_tc_common.cuh"
